@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <tuple>
+#include <type_traits>
 #include <stdint.h>
 #include <stdlib.h>
 #include <string.h>
@@ -204,6 +205,12 @@ struct SorsHandle {
     long long pcg_graph_kernels = 0;  // kernel nodes of the captured chunk
     int64_t n_hess_evals = 0, n_grad_evals = 0;  // system evaluations with / without the Hessian
     bool graph_failed = false;
+
+    // one-launch PCG (ensure_resident): 0 not looked at, 1 planned, -1 not for this mesh
+    int res_state = 0;
+    ResidentPlan res;
+    unsigned long long *res_zg = nullptr, *res_box = nullptr;
+    unsigned* res_epoch = nullptr;
 
     double prev_gnorm = -1.0;
     // PCG directions with non-positive curvature met during the last step:
@@ -962,8 +969,175 @@ void coarse_rate_check(SorsHandle* h, bool refreshed) {
     }
 }
 
+// Plan of the one-launch PCG (pcg_resident.cu), made at the first solve that
+// could use it: the row ranges, their border columns and local column indices.
+int ensure_resident(SorsHandle* h) {
+    if (h->res_state != 0) return SORS_OK;
+    h->res_state = -1;
+    const int N = h->N;
+    const int hs = (int)hsize(h);
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) return SORS_OK;
+    // a handle whose grids are capped takes the same share of the SMs
+    int gmax = std::min(sms, kResidentMaxBlocks);
+    if (h->s.max_blocks > 0) gmax = std::min(gmax, std::max(1, h->s.max_blocks * kResidentMaxBlocks / kRedBlocks));
+    const size_t bytes = (size_t)h->nnzb * 9 * hs;
+    ResidentPlan pl;
+    // One cluster up to 3.3 MB of matrix: its exchanges are three times cheaper,
+    // but 16 SMs hold and multiply the whole matrix.  Measured per iteration
+    // (cluster / grid): FP32 tets 2,744 nodes 3.7 / 5.3 us, 6,859 nodes (3.5 MB)
+    // 5.8 / 6.2 us; FP64 tets 1,000 nodes 4.0 / 6.2 us, 3,375 nodes (3.4 MB) 6.3 /
+    // 6.5 us, 4,225 nodes 7.6 / 6.5 us; FP64 hexes 891 nodes 13.6 / 18.1 us per
+    // adjoint iteration, 2,025 nodes 18.2 / 19.4 us.
+    pl.cluster = (N <= 16 * kResidentThreads && bytes <= ((size_t)16 * 200 << 10)) ? 1 : 0;
+    // Grid: 64 blocks, more where a block's rows would not have a lane group each.
+    // A sum over 148 blocks takes 2.2 us, over 64 1.4 us; 4,225 FP64 nodes per
+    // step: 148 blocks 5.6 ms, 96 5.0, 64 5.1, 36 5.4; 10,648 FP32 nodes per three
+    // steps: 148 blocks 48 ms, 96 44, 64 41, 36 50.
+    const int per = hs == 4 ? 160 : 128;
+    pl.G = pl.cluster ? std::max(1, std::min(16, (N + 31) / 32))
+                      : std::max(1, std::min({gmax, (N + 15) / 16, std::max(64, (N + per - 1) / per)}));
+    // ranges of about equal numbers of matrix blocks
+    std::vector<int> row0(pl.G + 1, 0);
+    row0[pl.G] = N;
+    for (int b = 1; b < pl.G; b++)
+        row0[b] = std::max(row0[b - 1], (int)(std::lower_bound(h->row_ptr_h.begin(), h->row_ptr_h.end(),
+                                              (int)(h->nnzb * b / pl.G)) - h->row_ptr_h.begin()));
+    std::vector<int> owner(N), halo, halo_ptr(pl.G + 1, 0);
+    for (int b = 0; b < pl.G; b++) {
+        pl.max_rows = std::max(pl.max_rows, row0[b + 1] - row0[b]);
+        for (int i = row0[b]; i < row0[b + 1]; i++) owner[i] = b;
+    }
+    if (pl.max_rows > kResidentThreads) return SORS_OK;
+    // lanes per row: as many as give every row of the range a group of its own;
+    // blocks per lane: what a tet row (15 blocks) or a hex row (27) needs of them
+    const int mean = (int)(h->nnzb / std::max(1, N));
+    pl.lpr = pl.max_rows <= kResidentThreads / 8 ? 8 : (pl.max_rows <= kResidentThreads / 4 || hs == 8 ? 4 : 2);
+    if (mean > 18 && pl.lpr == 2) pl.lpr = 4;
+    pl.reg = pl.lpr == 8 ? (mean > 18 ? 4 : 2) : (pl.lpr == 4 ? 4 : 8);
+    const int NG = kResidentThreads / pl.lpr;
+    std::vector<int> over((size_t)N + pl.G);
+    for (int b = 0; b < pl.G; b++) {
+        int* ov = over.data() + row0[b] + b;
+        ov[0] = 0;
+        for (int i = row0[b]; i < row0[b + 1]; i++) {
+            const int len = h->row_ptr_h[i + 1] - h->row_ptr_h[i], k = i - row0[b];
+            ov[k + 1] = ov[k] + (k < NG ? std::max(0, len - pl.lpr * pl.reg) : len);
+        }
+        pl.max_over = std::max(pl.max_over, ov[row0[b + 1] - row0[b]]);
+    }
+    std::vector<uint16_t> lcol((size_t)h->nnzb);
+    std::vector<int> seen(N, -1), local(N, 0);
+    for (int b = 0; b < pl.G; b++) {
+        const int a0 = row0[b], a1 = row0[b + 1];
+        const size_t first = halo.size();
+        for (int k = h->row_ptr_h[a0]; k < h->row_ptr_h[a1]; k++) {
+            const int j = h->col_h[k];
+            if (j >= a0 && j < a1) {
+                lcol[k] = (uint16_t)(j - a0);
+                continue;
+            }
+            if (seen[j] != b) {
+                seen[j] = b;
+                local[j] = (int)(halo.size() - first) + a1 - a0;
+                halo.push_back(j);
+            }
+            if (local[j] > 65535) return SORS_OK;
+            lcol[k] = (uint16_t)local[j];
+        }
+        halo_ptr[b + 1] = (int)halo.size();
+        pl.max_halo = std::max(pl.max_halo, (int)(halo.size() - first));
+        pl.max_cols = std::max(pl.max_cols, (int)(halo.size() - first) + a1 - a0);
+    }
+    std::vector<int> push_ptr, push;
+    if (pl.cluster) {
+        push_ptr.assign(N + 1, 0);
+        for (int j : halo) push_ptr[j + 1]++;
+        for (int i = 0; i < N; i++) push_ptr[i + 1] += push_ptr[i];
+        push.resize(halo.size());
+        std::vector<int> pos(push_ptr.begin(), push_ptr.end() - 1);
+        for (int b = 0; b < pl.G; b++)
+            for (int k = halo_ptr[b]; k < halo_ptr[b + 1]; k++) push[pos[halo[k]]++] = b << 16 | (k - halo_ptr[b]);
+        for (int b = 0; b < pl.G; b++) pl.max_push = std::max(pl.max_push, push_ptr[row0[b + 1]] - push_ptr[row0[b]]);
+    }
+    const size_t fixed = resident_smem(pl, hs, 0);
+    if (fixed > (size_t)kResidentSmem) return SORS_OK;
+    pl.res_blocks = std::min(pl.max_over, (int)((kResidentSmem - fixed) / (9 * (size_t)hs)));
+    pl.smem_bytes = (int)resident_smem(pl, hs, pl.res_blocks);
+    if (!pl.cluster && 2 * pl.res_blocks < pl.max_over) return SORS_OK;
+    // one allocation: z, mailboxes and epoch (zeroed), then the plan's arrays
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t zb = pl.cluster ? 0 : up((size_t)N * (hs == 4 ? 4 : 6) * 8);
+    const size_t bb = pl.cluster ? 0 : up((size_t)pl.G * 6 * kResidentBoxEntries * 8);
+    std::vector<int> ints;
+    auto put = [&](const std::vector<int>& v) {
+        const size_t at = ints.size();
+        ints.insert(ints.end(), v.begin(), v.end());
+        return at;
+    };
+    const size_t i_row0 = put(row0), i_hp = put(halo_ptr), i_halo = put(halo), i_over = put(over),
+                 i_pp = put(push_ptr), i_push = put(push);
+    const size_t ib = up(ints.size() * sizeof(int));
+    char* base = nullptr;
+    int st;
+    if ((st = dalloc(h, (void**)&base, zb + bb + 256 + ib + lcol.size() * 2))) return st;
+    CK(cudaMemsetAsync(base, 0, zb + bb + 256, h->stream));
+    h->res_zg = (unsigned long long*)base;
+    h->res_box = (unsigned long long*)(base + zb);
+    h->res_epoch = (unsigned*)(base + zb + bb);
+    char* ibase = base + zb + bb + 256;
+    CK(h2d(h, ibase, ints.data(), ints.size() * sizeof(int)));
+    CK(h2d(h, ibase + ib, lcol.data(), lcol.size() * 2));
+    const int* id = (const int*)ibase;
+    pl.row0 = id + i_row0; pl.halo_ptr = id + i_hp; pl.halo = id + i_halo; pl.over = id + i_over;
+    pl.push_ptr = id + i_pp; pl.push = id + i_push;
+    pl.lcol = (const uint16_t*)(ibase + ib);
+    h->res = pl;
+    h->res_state = 1;
+    return SORS_OK;
+}
+
+// The solve as one launch; *ran = false when it cannot be launched here.
+template <typename VT>
+int pcg_resident(SorsHandle* h, double eta, double abs_tol, const double* g, bool* ran) {
+    ResidentArgs<VT> a;
+    a.row_ptr = h->row_ptr; a.diag_slot = h->diag_slot; a.H = (const VT*)h->H; a.g = g ? g : h->g;
+    a.x = (VT*)h->x; a.p0 = (VT*)h->p0; a.p1 = (VT*)h->p1; a.zg = h->res_zg; a.box = h->res_box;
+    a.eta2 = eta * eta; a.abs_tol2 = abs_tol * abs_tol; a.maxit = h->s.pcg_max_iter;
+    a.pflag = h->proj_flag; a.pn = h->proj_n; a.epoch = h->res_epoch; a.sc = h->sc;
+    *ran = launch_pcg_resident<VT>(h->res, a, h->stream) == 0;
+    if (!*ran) {
+        cudaGetLastError();
+        h->res_state = -1;
+        return SORS_OK;
+    }
+    CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    if (h->sc_host->status & kFlagTimeout) return fail(SORS_ERR_CUDA, "the PCG blocks did not meet within the limit");
+    return SORS_OK;
+}
+
 template <typename HT, typename VT>
 int pcg_solve(SorsHandle* h, double eta, double abs_tol, int* iters, const double* g = nullptr) {
+    static_assert(std::is_same<HT, VT>::value, "PCG vectors have the matrix's type");
+    const bool plain = h->batch.nmem <= 1 && !(h->s.two_level && h->cargs.nc > 0);
+    bool ran = false;
+    if (plain) {
+        h->tl_active = false;
+        int st = ensure_resident(h);
+        if (st) return st;
+        if (h->res_state == 1 && (st = pcg_resident<VT>(h, eta, abs_tol, g, &ran))) return st;
+    }
+    if (ran) {
+        *iters = h->sc_host->it;
+        if (h->sc_host->breakdown) {
+            int st = record_curvature<VT>(h);
+            if (st) return st;
+            if (h->sc_host->it == 0 && !(h->s.project_spd == 2 && !h->proj_fallback))
+                return fail(SORS_ERR_PCG_BREAKDOWN, "PCG breakdown: the Hessian is not positive definite");
+        }
+        return SORS_OK;
+    }
     launch_block_jacobi<HT, VT>(h->N, h->row_ptr, h->diag_slot, (const HT*)h->H, h->nnzb, (VT*)h->Minv, h->stream);
     if (h->batch.nmem > 1) return pcg_solve_members<HT, VT>(h, eta, abs_tol, iters, g);
     // the two-level preconditioner: with a constraint projection (SQP, adjoint)

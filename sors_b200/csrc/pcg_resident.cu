@@ -1,0 +1,648 @@
+// pcg_resident.cu -- a whole block-Jacobi PCG solve in one launch, with the
+// matrix resident in registers and shared memory.
+//
+// What bounds the solve of a mesh up to some tens of thousands of nodes is not
+// its bytes: the matrix of 4,225 nodes is 4.3 MB in FP64 and sits in L2, but an
+// iteration as three launches (p, SpMV with p.q, update with r.z) took 15-17 us
+// of launch gaps, cold starts and two grid-wide reductions through a last
+// block.  Here the thread blocks stay: each owns a contiguous range of rows
+// (the locality numbering makes neighbouring rows neighbouring nodes), loads
+// its CSR blocks once, and iterates until the solve ends.  An iteration
+// exchanges z at the range's border and two sums, nothing else:
+//
+//   p = z + beta p     own and border columns (a border column's p is formed by
+//                      every range that reads it, from the same z: same bits)
+//   q = A p, p.q       lanes of a group share a row, shuffles add it
+//   [sum]  alpha       x += alpha p, r -= alpha q, z = M^-1 r, publish z
+//   [sum]  beta        r.z, r.r
+//
+// Matrix: a group of LPR lanes holds the first R * LPR blocks of its row in
+// registers (the register file is the largest and fastest memory of an SM, and
+// nine values per block from shared memory at 2-3 way bank conflicts were two
+// thirds of an iteration); what does not fit, longer rows and the rows beyond
+// one per group, is in shared memory, and past that is read through L2.
+//
+// Two forms of the exchange:
+//   cluster  up to 16 blocks of one cluster: partial sums and border z are
+//            pushed into the readers' shared memory (st.async), each site's
+//            mbarrier counts the bytes.  A reader waits on its own mbarrier.
+//   grid     a cooperative launch over the SMs: every block pushes its partial
+//            sum into every block's mailbox in global memory and polls its own,
+//            z goes through global memory.  Each 64-bit word carries 32 bits of
+//            the value and the 32-bit epoch, so a word says by itself whether it
+//            has arrived: no fence, no atomic, no flag.  (Polling one shared set
+//            of slots instead took 4-5 us per sum: 148 readers on 37 lines.)
+//
+// All sums run in a fixed order, so a solve is bit-reproducible.
+//
+// Measured, whole iteration (three launches before -> here): cluster, 1,728
+// FP32 nodes 15 -> 3.8 us; grid, 4,225 FP64 nodes 15 -> 6.4 us, 10,648 FP32 nodes
+// 17 -> 6.2 us, 18,921 FP64 hex nodes (33 MB of matrix) 25 -> 10.8 us.  What bounds
+// it now: the two sums' round trips through L2 (1.4 us each over 64 blocks, of
+// which 1.2 us is one store and one load) or, in a cluster, latency of the
+// dependent FP64 steps (about 1,000 cycles a sum, 1,100 a product).
+#include <cooperative_groups.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "fem_math.cuh"
+#include "sors_internal.h"
+
+namespace cg = cooperative_groups;
+
+namespace sors {
+
+namespace {
+
+constexpr int kT = kResidentThreads;
+constexpr int kWarps = kT / 32;
+constexpr int kBoxes = kResidentBoxEntries;  // mailbox entries: five per polling lane
+constexpr int kPollLimit = 1 << 21;          // about a second
+static_assert(kResidentMaxBlocks <= kBoxes && kBoxes % 32 == 0, "a lane polls kBoxes / 32 entries");
+typedef unsigned long long u64;
+
+// values per node of a column's p: one 16-byte load (FP32), three 8-byte loads (FP64)
+template <typename VT>
+struct Lay {
+    static constexpr int P = sizeof(VT) == 4 ? 4 : 3;
+    static constexpr int Z = sizeof(VT) == 4 ? 4 : 6;  // 64-bit words of a published z (grid form)
+};
+
+// Byte offsets of a block's shared memory, the same in every block of a launch.
+struct Off {
+    int sp, sq, sm, sx, sz, sov, sgb, shalo, spp, spush, scol, sval;
+};
+template <typename VT>
+__host__ __device__ inline Off offsets(const ResidentPlan& pl) {
+    auto up = [](int b) { return (b + 15) & ~15; };
+    Off o;
+    int at = 1024;  // Scratch
+    o.sp = at; at = up(at + pl.max_cols * Lay<VT>::P * (int)sizeof(VT));
+    o.sq = at; at = up(at + pl.max_rows * 3 * (int)sizeof(VT));
+    o.sm = at; at = up(at + pl.max_rows * 9 * (int)sizeof(VT));
+    o.sx = at; at = up(at + pl.max_rows * 9 * (int)sizeof(VT));
+    o.sz = at; at = up(at + (pl.cluster ? pl.max_halo * 4 * (int)sizeof(VT) : 0));
+    o.sov = at; at = up(at + (pl.max_rows + 1) * 4);
+    o.sgb = at; at = up(at + pl.max_rows * 4);
+    o.shalo = at; at = up(at + (pl.cluster ? 0 : pl.max_halo * 4));
+    o.spp = at; at = up(at + (pl.cluster ? (pl.max_rows + 1) * 4 : 0));
+    o.spush = at; at = up(at + (pl.cluster ? pl.max_push * 4 : 0));
+    o.scol = at; at = up(at + pl.max_over * 2);
+    o.sval = at;
+    return o;
+}
+
+__device__ __forceinline__ void st_words(u64* p, u64 a, u64 b) {
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ void ld_words(const u64* p, u64& a, u64& b) {
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ u64 tagged(unsigned v, unsigned epoch) { return ((u64)epoch << 32) | v; }
+__device__ __forceinline__ bool has(u64 w, unsigned epoch) { return (unsigned)(w >> 32) == epoch; }
+__device__ __forceinline__ double join(u64 lo, u64 hi) {
+    return __longlong_as_double((long long)((hi << 32) | (lo & 0xffffffffull)));
+}
+__device__ __forceinline__ void split(double v, unsigned epoch, u64& lo, u64& hi) {
+    const u64 b = (u64)__double_as_longlong(v);
+    lo = tagged((unsigned)b, epoch);
+    hi = tagged((unsigned)(b >> 32), epoch);
+}
+
+// cluster form: the address of `local` in block `rank`, and pushes that count
+// their bytes on that block's mbarrier
+__device__ __forceinline__ unsigned remote(const void* local, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void push(unsigned dst, unsigned bar, double a) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(dst), "d"(a),
+                 "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void push(unsigned dst, unsigned bar, double a, double b) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                 "d"(a), "d"(b), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void push(unsigned dst, unsigned bar, float a, float b, float c) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
+                     dst),
+                 "f"(a), "f"(b), "f"(c), "f"(0.0f), "r"(bar)
+                 : "memory");
+}
+
+// Fixed scratch at the start of the block's shared memory.
+struct Scratch {
+    u64 bar[2];             // cluster form: one mbarrier per reduction site
+    double part[kWarps][2];
+    double tot[2];
+    int abort, pad;
+    alignas(16) double slot[2][16][2];  // cluster form: the blocks' partial sums, by reduction site (16-byte pushes)
+};
+static_assert(sizeof(Scratch) <= 1024, "fixed scratch");
+
+// Sums v, already summed within each warp, over all blocks; every thread gets
+// the totals.  SITE 0: p.q, 1: r.z and r.r (and border z).  The sites alternate,
+// so a slot or mailbox entry is written again only after every block has read
+// it.  halo_bytes: border z the block receives with site 1 (cluster form).
+// False: something did not arrive within the poll limit.
+template <int SITE, bool CL>
+__device__ __forceinline__ bool all_sum(double (&v)[SITE + 1], Scratch* sh, int G, unsigned epoch, u64* box,
+                                        unsigned parity, int halo_bytes) {
+    constexpr int NS = SITE + 1;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, me = blockIdx.x;
+    if (l == 0)
+#pragma unroll
+        for (int s = 0; s < NS; s++) sh->part[w][s] = v[s];
+    __syncthreads();
+    if (w == 0) {
+#pragma unroll
+        for (int s = 0; s < NS; s++) v[s] = sh->part[l & (kWarps - 1)][s];
+#pragma unroll
+        for (int o = kWarps / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int s = 0; s < NS; s++) v[s] += __shfl_xor_sync(0xffffffffu, v[s], o);
+    }
+    if constexpr (CL) {
+        const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh->bar[SITE]);
+        if (w == 0) {
+            if (l == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                             "r"(G * 8 * NS + halo_bytes)
+                             : "memory");
+            __syncwarp();
+            if (l < G) {
+                const unsigned dst = remote(&sh->slot[SITE][me][0], l), rb = remote(&sh->bar[SITE], l);
+                if constexpr (NS == 1) push(dst, rb, v[0]);
+                else push(dst, rb, v[0], v[1]);
+            }
+        }
+        unsigned got = 0;
+        for (int n = 0; n < kPollLimit && !got; n++)
+            asm volatile(
+                "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                " selp.u32 %0, 1, 0, p;\n}"
+                : "=r"(got)
+                : "r"(bar), "r"(parity)
+                : "memory");
+        if (!got) sh->abort = 1;
+        // 16 values: a lane each (twice per warp), four shuffles
+#pragma unroll
+        for (int s = 0; s < NS; s++) v[s] = (l & 15) < G ? sh->slot[SITE][l & 15][s] : 0.0;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+            for (int s = 0; s < NS; s++) v[s] += __shfl_xor_sync(0xffffffffu, v[s], o);
+        return true;
+    } else {
+        if (w == 0) {
+            constexpr int J = kBoxes / 32;
+            constexpr int kSite1 = 2 * kBoxes, kBox = 6 * kBoxes;  // words: site 0, then site 1
+            u64 lo[NS], hi[NS];
+#pragma unroll
+            for (int s = 0; s < NS; s++) split(v[s], epoch, lo[s], hi[s]);
+            const size_t at = SITE ? kSite1 : 0;
+#pragma unroll
+            for (int j = 0; j < J; j++)
+                if (l + 32 * j < G)
+#pragma unroll
+                    for (int s = 0; s < NS; s++)
+                        st_words(box + (size_t)(l + 32 * j) * kBox + at + (size_t)me * 2 * NS + 2 * s, lo[s], hi[s]);
+            // a lane's entries are loaded together, so a round of polls is one trip to L2
+            const u64* q = box + (size_t)me * kBox + at + (size_t)l * 2 * NS;
+            u64 a[J][NS], b[J][NS];
+            bool ok;
+            int n = 0;
+            do {
+                ok = true;
+#pragma unroll
+                for (int j = 0; j < J; j++)
+                    if (l + 32 * j < G)
+#pragma unroll
+                        for (int s = 0; s < NS; s++) ld_words(q + 64 * NS * j + 2 * s, a[j][s], b[j][s]);
+#pragma unroll
+                for (int j = 0; j < J; j++)
+                    if (l + 32 * j < G)
+#pragma unroll
+                        for (int s = 0; s < NS; s++) ok = ok && has(a[j][s], epoch) && has(b[j][s], epoch);
+                ok = __all_sync(0xffffffffu, ok);  // the warp stays together
+            } while (!ok && ++n < kPollLimit);
+            double t[NS];
+#pragma unroll
+            for (int s = 0; s < NS; s++) t[s] = 0.0;
+#pragma unroll
+            for (int j = 0; j < J; j++)
+                if (l + 32 * j < G)
+#pragma unroll
+                    for (int s = 0; s < NS; s++) t[s] += join(a[j][s], b[j][s]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int s = 0; s < NS; s++) t[s] += __shfl_xor_sync(0xffffffffu, t[s], o);
+            if (l == 0) {
+#pragma unroll
+                for (int s = 0; s < NS; s++) sh->tot[s] = t[s];
+                if (!ok) sh->abort = 1;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < NS; s++) v[s] = sh->tot[s];
+        return sh->abort == 0;
+    }
+}
+
+template <typename VT>
+__device__ __forceinline__ void project(unsigned f, const double4* pn, VT (&y)[3]) {
+    if (!f) return;
+    if (f & 1u) y[0] = VT(0);
+    if (f & 2u) y[1] = VT(0);
+    if (f & 4u) y[2] = VT(0);
+    if (f & 8u) {
+        const double4 n = *pn;
+        const VT d = (VT)n.x * y[0] + (VT)n.y * y[1] + (VT)n.z * y[2];
+        y[0] -= d * (VT)n.x;
+        y[1] -= d * (VT)n.y;
+        y[2] -= d * (VT)n.z;
+    }
+}
+
+template <typename VT>
+__device__ __forceinline__ void ld_p(const VT* p, VT& a, VT& b, VT& c) {
+    if constexpr (sizeof(VT) == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(p);
+        a = t.x; b = t.y; c = t.z;
+    } else {
+        a = p[0]; b = p[1]; c = p[2];
+    }
+}
+
+// A loaded value stays in its register: the compiler may not load it again.
+__device__ __forceinline__ void keep(float& v) { asm volatile("" : "+f"(v)); }
+__device__ __forceinline__ void keep(double& v) { asm volatile("" : "+d"(v)); }
+
+template <typename VT, int LPR, int R, bool CL>
+__global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, ResidentArgs<VT> a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int P = Lay<VT>::P, Z = Lay<VT>::Z;
+    constexpr int NG = kT / LPR;  // groups of lanes
+    Scratch* sh = reinterpret_cast<Scratch*>(smem);
+    const Off o = offsets<VT>(pl);
+    VT* sp = reinterpret_cast<VT*>(smem + o.sp);
+    VT* sq = reinterpret_cast<VT*>(smem + o.sq);
+    VT* sm = reinterpret_cast<VT*>(smem + o.sm);
+    VT* sz = reinterpret_cast<VT*>(smem + o.sz);
+    int* sov = reinterpret_cast<int*>(smem + o.sov);
+    int* sgb = reinterpret_cast<int*>(smem + o.sgb);
+    int* shalo = reinterpret_cast<int*>(smem + o.shalo);
+    int* spp = reinterpret_cast<int*>(smem + o.spp);
+    int* spush = reinterpret_cast<int*>(smem + o.spush);
+    uint16_t* scol = reinterpret_cast<uint16_t*>(smem + o.scol);
+    VT* sval = reinterpret_cast<VT*>(smem + o.sval);
+    const int t = threadIdx.x, lane = t & 31, G = gridDim.x, me = blockIdx.x;
+    const int r0 = pl.row0[me], nr = pl.row0[me + 1] - r0;
+    const int h0 = pl.halo_ptr[me], nh = pl.halo_ptr[me + 1] - h0;
+    unsigned epoch = CL ? 0u : *(volatile const unsigned*)a.epoch;
+    if (t == 0) {
+        sh->abort = 0;
+        if constexpr (CL)
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&sh->bar[k]))
+                             : "memory");
+        if constexpr (CL) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // every block runs, its barriers set up, before any pushes into another's shared memory
+    if constexpr (CL) cg::this_cluster().sync();
+
+    // matrix: the group's first row in registers ...
+    const int g = t / LPR, sl = t % LPR;
+    VT hv[R][9];
+    int hc[R];
+    {
+        const int gb = g < nr ? a.row_ptr[r0 + g] : 0, len = g < nr ? a.row_ptr[r0 + g + 1] - gb : 0;
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const int k = sl + LPR * j;
+            hc[j] = k < len ? P * (int)pl.lcol[gb + k] : 0;
+#pragma unroll
+            for (int e = 0; e < 9; e++) {
+                hv[j][e] = k < len ? __ldg(a.H + 9 * (size_t)(gb + k) + e) : VT(0);
+                keep(hv[j][e]);
+            }
+        }
+    }
+    // ... the rest of its blocks and the rows beyond NG in shared memory, while it lasts
+    for (int i = t; i <= nr; i += kT) sov[i] = pl.over[r0 + me + i];
+    __syncthreads();
+    for (int i = t >> 5; i < nr; i += kWarps) {
+        const int gb = a.row_ptr[r0 + i + 1] - (sov[i + 1] - sov[i]);  // first block not in registers
+        if (lane == 0) sgb[i] = gb;
+        const int n = sov[i + 1] - sov[i], nres = min(max(pl.res_blocks - sov[i], 0), n);
+        for (int k = lane; k < n; k += 32) scol[sov[i] + k] = pl.lcol[gb + k];
+        for (int k = lane; k < 9 * nres; k += 32) sval[9 * sov[i] + k] = __ldg(a.H + 9 * (size_t)gb + k);
+    }
+    if constexpr (CL) {
+        const int q0 = pl.push_ptr[r0], np = pl.push_ptr[r0 + nr] - q0;
+        for (int i = t; i <= nr; i += kT) spp[i] = pl.push_ptr[r0 + i] - q0;
+        for (int k = t; k < np; k += kT) spush[k] = pl.push[q0 + k];
+    } else {
+        for (int k = t; k < nh; k += kT) shalo[k] = pl.halo[h0 + k];
+    }
+    for (int k = t; k < (nr + nh) * P; k += kT) sp[k] = VT(0);
+
+    // one thread per row: x, r, z and the inverse diagonal block (as k_block_jacobi), in
+    // shared memory (a row's nine values are an odd stride: no bank conflicts), so that
+    // the registers are left to the matrix
+    VT* M = sm + 9 * t;
+    VT* x = reinterpret_cast<VT*>(smem + o.sx) + 9 * t;
+    VT *rs = x + 3, *zs = x + 6;
+    unsigned pf = 0;
+    const size_t row = (size_t)r0 + t;
+    if (t < nr) {
+        double d[9], c[9];
+        const VT* hd = a.H + 9 * (size_t)a.diag_slot[row];
+#pragma unroll
+        for (int k = 0; k < 9; k++) d[k] = (double)hd[k];
+        d[1] = d[3]; d[2] = d[6]; d[5] = d[7];
+        cof3(d, c);
+        const double det = d[0] * c[0] + d[1] * c[1] + d[2] * c[2];
+        const bool inv = det != 0.0 && det == det;
+        const double id = 1.0 / det;
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+#pragma unroll
+            for (int m = 0; m < 3; m++)
+                M[k * 3 + m] = inv ? (VT)(c[m * 3 + k] * id) : (VT)(k == m ? 1.0 : 0.0);
+        if (a.pflag) pf = a.pflag[row];
+        VT r[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) r[k] = (VT)(-a.g[3 * row + k]);
+        project<VT>(pf, a.pn + row, r);
+#pragma unroll
+        for (int k = 0; k < 3; k++) { x[k] = VT(0); rs[k] = r[k]; }
+    }
+    __syncthreads();
+
+    // z = M^-1 r, published with the coming site-1 sum; r.z and r.r of the warp
+    auto precondition = [&](double (&acc)[2]) {
+        acc[0] = acc[1] = 0.0;
+        if (t < nr) {
+            VT z[3];
+            const VT r[3] = {rs[0], rs[1], rs[2]};
+#pragma unroll
+            for (int k = 0; k < 3; k++) z[k] = M[k * 3] * r[0] + M[k * 3 + 1] * r[1] + M[k * 3 + 2] * r[2];
+            project<VT>(pf, a.pn + row, z);
+#pragma unroll
+            for (int k = 0; k < 3; k++) zs[k] = z[k];
+            if constexpr (CL) {
+                for (int k = spp[t]; k < spp[t + 1]; k++) {
+                    const int d = spush[k];
+                    const unsigned dst = remote(sz + 4 * (d & 0xffff), d >> 16), rb = remote(&sh->bar[1], d >> 16);
+                    if constexpr (sizeof(VT) == 4) {
+                        push(dst, rb, z[0], z[1], z[2]);
+                    } else {
+                        push(dst, rb, z[0], z[1]);
+                        push(dst + 16, rb, z[2]);
+                    }
+                }
+            } else {
+                u64 w[Z];
+                if constexpr (sizeof(VT) == 4) {
+#pragma unroll
+                    for (int k = 0; k < 3; k++) w[k] = tagged(__float_as_uint((float)z[k]), epoch + 1);
+                    w[3] = w[2];
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 3; k++) split((double)z[k], epoch + 1, w[2 * k], w[2 * k + 1]);
+                }
+#pragma unroll
+                for (int k = 0; k < Z; k += 2) st_words(a.zg + Z * row + k, w[k], w[k + 1]);
+            }
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                acc[0] += (double)r[k] * (double)z[k];
+                acc[1] += (double)r[k] * (double)r[k];
+            }
+        }
+        if ((t & ~31) < nr) {  // a warp with rows
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1) {
+                acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], s);
+                acc[1] += __shfl_xor_sync(0xffffffffu, acc[1], s);
+            }
+        }
+    };
+    constexpr int kZBytes = sizeof(VT) == 4 ? 16 : 24;
+    unsigned parity = 0;  // of both sites: they complete alternately, site 1 first
+    double acc[2];
+    precondition(acc);
+    bool ok = all_sum<1, CL>(acc, sh, G, ++epoch, a.box, 0u, nh * kZBytes);
+    double rz = acc[0], rr = acc[1], pq = 0.0, alpha = 0.0, beta = 0.0;
+    const double bnorm2 = rr;
+    const double te = a.eta2 * rr, tol2 = te > a.abs_tol2 ? te : a.abs_tol2;
+    int it = 0, breakdown = 0;
+    bool done = !ok || rr <= tol2 || a.maxit <= 0;
+    // threads without a row take the border columns first
+    const int nru = (nr + 31) & ~31;
+    const int th = t >= nru ? t - nru : t + kT - nru;
+    while (!done) {
+        // p at the range's own and border columns
+        const VT bt = (VT)beta;
+        if (t < nr) {
+            VT* pc = sp + P * t;
+#pragma unroll
+            for (int k = 0; k < 3; k++) pc[k] = zs[k] + bt * pc[k];
+        }
+        for (int k = th; k < nh; k += kT) {
+            VT zz[3];
+            if constexpr (CL) {
+#pragma unroll
+                for (int m = 0; m < 3; m++) zz[m] = sz[4 * k + m];
+            } else {
+                const u64* q = a.zg + Z * (size_t)shalo[k];
+                u64 w[Z];
+                bool here;
+                int n = 0;
+                do {
+                    here = true;
+#pragma unroll
+                    for (int m = 0; m < Z; m += 2) ld_words(q + m, w[m], w[m + 1]);
+#pragma unroll
+                    for (int m = 0; m < Z; m++) here = here && has(w[m], epoch);
+                } while (!here && ++n < kPollLimit);
+                if (!here) sh->abort = 1;
+                if constexpr (sizeof(VT) == 4) {
+#pragma unroll
+                    for (int m = 0; m < 3; m++) zz[m] = (VT)__uint_as_float((unsigned)w[m]);
+                } else {
+#pragma unroll
+                    for (int m = 0; m < 3; m++) zz[m] = (VT)join(w[2 * m], w[2 * m + 1]);
+                }
+            }
+            VT* pc = sp + P * (nr + k);
+#pragma unroll
+            for (int m = 0; m < 3; m++) pc[m] = zz[m] + bt * pc[m];
+        }
+        // a block barrier does not bring lanes together that left the loop apart,
+        // and a warp in pieces runs what follows once per piece
+        __syncwarp();
+        __syncthreads();
+        double d1[1] = {0.0};
+        for (int base = 0; base + (t & ~31) / LPR < nr; base += NG) {
+            const int i = base + g;
+            VT a0 = VT(0), a1 = VT(0), a2 = VT(0), p0, p1, p2;
+            if (base == 0) {
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    ld_p<VT>(sp + hc[j], p0, p1, p2);
+                    a0 += hv[j][0] * p0 + hv[j][1] * p1 + hv[j][2] * p2;
+                    a1 += hv[j][3] * p0 + hv[j][4] * p1 + hv[j][5] * p2;
+                    a2 += hv[j][6] * p0 + hv[j][7] * p1 + hv[j][8] * p2;
+                }
+            }
+            if (i < nr) {
+                const int o0 = sov[i], n = sov[i + 1] - o0;
+                for (int k = sl; k < n; k += LPR) {
+                    VT h[9];
+                    if (o0 + k < pl.res_blocks) {
+#pragma unroll
+                        for (int e = 0; e < 9; e++) h[e] = sval[9 * (o0 + k) + e];
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 9; e++) h[e] = __ldg(a.H + 9 * (size_t)(sgb[i] + k) + e);
+                    }
+                    ld_p<VT>(sp + P * (int)scol[o0 + k], p0, p1, p2);
+                    a0 += h[0] * p0 + h[1] * p1 + h[2] * p2;
+                    a1 += h[3] * p0 + h[4] * p1 + h[5] * p2;
+                    a2 += h[6] * p0 + h[7] * p1 + h[8] * p2;
+                }
+            }
+#pragma unroll
+            for (int s = LPR / 2; s > 0; s >>= 1) {
+                a0 += __shfl_xor_sync(0xffffffffu, a0, s);
+                a1 += __shfl_xor_sync(0xffffffffu, a1, s);
+                a2 += __shfl_xor_sync(0xffffffffu, a2, s);
+            }
+            if (i < nr) {
+                if (sl == 0) { sq[3 * i] = a0; sq[3 * i + 1] = a1; sq[3 * i + 2] = a2; }
+                ld_p<VT>(sp + P * i, p0, p1, p2);
+                d1[0] += (double)p0 * (double)a0 + (double)p1 * (double)a1 + (double)p2 * (double)a2;
+            }
+        }
+        // every lane of a group has its rows' share of p.q: add the warp's groups
+#pragma unroll
+        for (int s = 16; s >= LPR; s >>= 1) d1[0] += __shfl_xor_sync(0xffffffffu, d1[0], s);
+        ok = all_sum<0, CL>(d1, sh, G, ++epoch, a.box, parity, 0);
+        if (!ok) break;
+        pq = d1[0];
+        if (!(pq > 0.0)) {
+            breakdown = 1;
+            break;
+        }
+        alpha = rz / pq;
+        const VT al = (VT)alpha;
+        if (t < nr) {
+            VT q[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                x[k] += al * sp[P * t + k];
+                q[k] = sq[3 * t + k];
+            }
+            project<VT>(pf, a.pn + row, q);
+#pragma unroll
+            for (int k = 0; k < 3; k++) rs[k] -= al * q[k];
+        }
+        precondition(acc);
+        parity ^= 1u;
+        ok = all_sum<1, CL>(acc, sh, G, ++epoch, a.box, parity, nh * kZBytes);
+        if (!ok) break;
+        beta = acc[0] / rz;
+        rz = acc[0];
+        rr = acc[1];
+        it++;
+        done = rr <= tol2 || it >= a.maxit || !(rr == rr);
+    }
+    if (t < nr) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) a.x[3 * row + k] = x[k];
+        if (breakdown) {
+            // the direction of non-positive curvature, where the caller looks for it
+            VT* pb = ((it & 1) ? a.p0 : a.p1) + 4 * row;
+#pragma unroll
+            for (int k = 0; k < 3; k++) pb[k] = sp[P * t + k];
+        }
+    }
+    // no block leaves while another may still push into its shared memory
+    if constexpr (CL) cg::this_cluster().sync();
+    else __syncthreads();
+    if (me == 0 && t == 0) {
+        DevScalars* sc = a.sc;
+        sc->rz = rz; sc->rr = rr; sc->bnorm2 = bnorm2; sc->tol2 = tol2; sc->pq = pq;
+        sc->alpha = breakdown ? 0.0 : alpha; sc->beta = beta;
+        sc->it = it; sc->maxit = a.maxit; sc->breakdown = breakdown; sc->done = 1;
+        if (sh->abort) sc->status |= kFlagTimeout;
+        if (!CL) *a.epoch = epoch;
+    }
+}
+
+template <typename VT, int LPR, int R, bool CL>
+int launch_one(const ResidentPlan& pl, const ResidentArgs<VT>& a, cudaStream_t st) {
+    auto kern = k_pcg_resident<VT, LPR, R, CL>;
+    static std::atomic<int> done[kMaxDevices];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= kMaxDevices || !done[dev].load(std::memory_order_relaxed)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmem);
+        if (e == cudaSuccess && CL) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return (int)e;
+        if (dev >= 0 && dev < kMaxDevices) done[dev].store(1, std::memory_order_relaxed);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pl.G);
+    cfg.blockDim = dim3(kT);
+    cfg.dynamicSmemBytes = pl.smem_bytes;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    if (CL) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = pl.G;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, pl, a);
+    if (e != cudaSuccess) return (int)e;
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    return 0;
+}
+
+template <typename VT, bool CL>
+int launch_shape(const ResidentPlan& pl, const ResidentArgs<VT>& a, cudaStream_t st) {
+    if (pl.lpr == 8) return pl.reg == 2 ? launch_one<VT, 8, 2, CL>(pl, a, st) : launch_one<VT, 8, 4, CL>(pl, a, st);
+    if constexpr (sizeof(VT) == 4)
+        if (pl.lpr == 2) return launch_one<VT, 2, 8, CL>(pl, a, st);
+    return launch_one<VT, 4, 4, CL>(pl, a, st);
+}
+
+}  // namespace
+
+// Shared memory of a plan's block with `res` matrix blocks in it.
+size_t resident_smem(const ResidentPlan& pl, int vsize, int res) {
+    const int at = vsize == 4 ? offsets<float>(pl).sval : offsets<double>(pl).sval;
+    return (size_t)at + 9 * (size_t)res * vsize;
+}
+
+template <typename VT>
+int launch_pcg_resident(const ResidentPlan& pl, const ResidentArgs<VT>& a, cudaStream_t st) {
+    return pl.cluster ? launch_shape<VT, true>(pl, a, st) : launch_shape<VT, false>(pl, a, st);
+}
+template int launch_pcg_resident<float>(const ResidentPlan&, const ResidentArgs<float>&, cudaStream_t);
+template int launch_pcg_resident<double>(const ResidentPlan&, const ResidentArgs<double>&, cudaStream_t);
+
+}  // namespace sors

@@ -173,6 +173,48 @@ void launch_bpcg_iter(const BatchArgs& b, const int* row_ptr, const int* col, co
                       const VT* z_in, const VT* p_old, VT* p_new, VT* qv, VT* x, VT* r, VT* z,
                       const uint8_t* pflag, const double4* pn, cudaStream_t st);
 
+// A whole block-Jacobi PCG solve in one launch (pcg_resident.cu): G blocks of
+// kResidentThreads threads, block b owning the rows [row0[b], row0[b + 1]).
+constexpr int kResidentThreads = 512;
+constexpr int kResidentMaxBlocks = 148;
+constexpr int kResidentBoxEntries = 160;
+constexpr int kResidentSmem = 232448;  // 227 KB, the most a block may have
+struct ResidentPlan {
+    int G = 0, cluster = 0;             // blocks; 1: one cluster, 0: a cooperative grid
+    int lpr = 8, reg = 2;               // lanes per row, matrix blocks per lane in registers
+    int max_rows = 0, max_cols = 0, max_halo = 0, max_over = 0, max_push = 0;  // largest of any block
+    int res_blocks = 0;                 // matrix blocks in shared memory, of those not in registers
+    int smem_bytes = 0;
+    const int* row0 = nullptr;          // G + 1
+    const int* halo_ptr = nullptr;      // G + 1
+    const int* halo = nullptr;          // border columns (nodes)
+    const int* over = nullptr;          // N + G: per block rows + 1, the matrix blocks not in registers before a row
+    const int* push_ptr = nullptr;      // N + 1, cluster: the blocks that read a row's z ...
+    const int* push = nullptr;          // ... as block << 16 | its border column
+    const uint16_t* lcol = nullptr;     // per CSR block: row of the range, or rows + border column
+};
+template <typename VT>
+struct ResidentArgs {
+    const int* row_ptr = nullptr;
+    const int* diag_slot = nullptr;
+    const VT* H = nullptr;
+    const double* g = nullptr;          // right-hand side -g
+    VT* x = nullptr;
+    VT *p0 = nullptr, *p1 = nullptr;    // receive the direction of a breakdown (by the parity of the iteration)
+    double eta2 = 0.0, abs_tol2 = 0.0;
+    int maxit = 0;
+    const uint8_t* pflag = nullptr;     // constraint projection (null: none)
+    const double4* pn = nullptr;
+    unsigned long long* zg = nullptr;   // grid form: published z, 4 (FP32) or 6 (FP64) words per node
+    unsigned long long* box = nullptr;  // grid form: mailboxes, 6 x kResidentBoxEntries words per block
+    unsigned* epoch = nullptr;          // grid form: the last epoch used
+    DevScalars* sc = nullptr;
+};
+size_t resident_smem(const ResidentPlan& pl, int vsize, int res);
+// Returns 0 or the CUDA error of the launch.
+template <typename VT>
+int launch_pcg_resident(const ResidentPlan& pl, const ResidentArgs<VT>& a, cudaStream_t st);
+
 // Caps the grid of every kernel launched from this thread (kernels.cu).
 void set_grid_cap(int blocks);
 
