@@ -186,7 +186,7 @@ struct SorsHandle {
     int tl_npairs = 0;
     int *tl_pair_ptr = nullptr;
     int2 *tl_items = nullptr, *tl_ab = nullptr;
-    double *tl_Ac = nullptr, *tl_yc = nullptr, *tl_rowk = nullptr, *tl_colk = nullptr;
+    double *tl_Ac = nullptr, *tl_yc = nullptr, *tl_diag = nullptr, *tl_work = nullptr;
     void* tl_Ainv = nullptr;
     int tl_ld = 0;                    // leading dimension of tl_Ainv (nc rounded up to 16 bytes)
     int tl_refreshes = 0;
@@ -211,6 +211,16 @@ struct SorsHandle {
     ResidentPlan res;
     unsigned long long *res_zg = nullptr, *res_box = nullptr;
     unsigned* res_epoch = nullptr;
+    // its two-level preconditioner: one aggregate per row range
+    CoarseArgs rcargs;
+    int rc_npairs = 0;
+    int* rc_pair_ptr = nullptr;
+    int2 *rc_items = nullptr, *rc_ab = nullptr;
+    double *rc_Ac = nullptr, *rc_diag = nullptr, *rc_work = nullptr;
+    void* rc_Ainv = nullptr;
+    bool rc_ready = false;
+    double rc_ref_rate = 0.0;
+    int tl_req = 0;  // settings.two_level as given (2: where it pays)
 
     double prev_gnorm = -1.0;
     // PCG directions with non-positive curvature met during the last step:
@@ -937,6 +947,17 @@ void keep_coarse_in_l2(SorsHandle* h, size_t bytes) {
     }
 }
 
+int setup_two_level(SorsHandle* h, const double* X);
+
+// The launch-per-kernel PCG's two-level preconditioner, when a solve first needs
+// it (sors_create sets it up for meshes beyond the one-launch PCG).
+int ensure_two_level(SorsHandle* h) {
+    if (!h->s.two_level || h->cargs.nc > 0) return SORS_OK;
+    std::vector<double> X((size_t)h->ndof);
+    CK(d2h(h, X.data(), h->X, sizeof(double) * X.size()));
+    return setup_two_level(h, X.data());
+}
+
 // The coarse operator P^T H P of the Hessian in h->H, inverted in place.
 template <typename HT, typename VT>
 int build_coarse(SorsHandle* h) {
@@ -944,11 +965,11 @@ int build_coarse(SorsHandle* h) {
     CK(cudaMemsetAsync(h->tl_Ac, 0, sizeof(double) * (size_t)nc * nc, h->stream));
     if (sizeof(HT) == 4)
         launch_coarse_galerkin_f(h->tl_npairs, h->tl_pair_ptr, h->tl_items, h->tl_ab, h->col, (const float*)h->H,
-                                 h->nnzb, h->cargs, h->tl_Ac, h->stream);
+                                 h->nnzb, h->cargs, h->tl_Ac, h->tl_diag, h->stream);
     else
         launch_coarse_galerkin_d(h->tl_npairs, h->tl_pair_ptr, h->tl_items, h->tl_ab, h->col, (const double*)h->H,
-                                 h->nnzb, h->cargs, h->tl_Ac, h->stream);
-    launch_coarse_invert(nc, h->tl_Ac, h->tl_rowk, h->tl_colk, h->stream);
+                                 h->nnzb, h->cargs, h->tl_Ac, h->tl_diag, h->stream);
+    launch_coarse_invert(nc, h->tl_Ac, h->tl_diag, h->tl_work, h->stream);
     launch_to_vt_pad<VT>(nc, h->tl_ld, h->tl_Ac, (VT*)h->tl_Ainv, h->stream);
     keep_coarse_in_l2(h, (size_t)nc * h->tl_ld * sizeof(VT));
     h->tl_ready = true;
@@ -959,14 +980,40 @@ int build_coarse(SorsHandle* h) {
 // Rebuilds the coarse operator when the iterations per decade of residual
 // reduction of a solve of two decades or more doubled against the first such
 // solve after the last rebuild.
-void coarse_rate_check(SorsHandle* h, bool refreshed) {
-    if (refreshed) h->tl_ref_rate = -1.0;
+void coarse_rate_check(SorsHandle* h, bool refreshed, double* ref_rate, bool* ready) {
+    if (refreshed) *ref_rate = -1.0;
     const DevScalars& sh = *h->sc_host;
-    if (h->tl_active && sh.it >= 8 && sh.rr > 0.0 && sh.bnorm2 >= 1e4 * sh.rr) {
+    if (sh.it >= 8 && sh.rr > 0.0 && sh.bnorm2 >= 1e4 * sh.rr) {
         const double rate = sh.it / (0.5 * log10(sh.bnorm2 / sh.rr));
-        if (h->tl_ref_rate <= 0.0) h->tl_ref_rate = rate;
-        else if (rate > 2.0 * h->tl_ref_rate) h->tl_ready = false;
+        if (*ref_rate <= 0.0) *ref_rate = rate;
+        else if (rate > 2.0 * *ref_rate) *ready = false;
     }
+}
+
+// Aggregate pairs and their Hessian blocks (counting sort by pair key): pair k
+// holds items [pair_ptr[k], pair_ptr[k + 1]), each (CSR block, its row).
+void coarse_pairs(const SorsHandle* h, const std::vector<int>& aid, int nagg, std::vector<int>& pair_ptr,
+                  std::vector<int2>& pair_ab, std::vector<int2>& items) {
+    const int N = h->N;
+    const long long nkeys = (long long)nagg * nagg;
+    std::vector<int> keycnt((size_t)nkeys, 0);
+    for (int i = 0; i < N; i++)
+        for (int b = h->row_ptr_h[i]; b < h->row_ptr_h[i + 1]; b++) keycnt[(size_t)aid[i] * nagg + aid[h->col_h[b]]]++;
+    pair_ptr.assign(1, 0);
+    pair_ab.clear();
+    std::vector<int> keypos((size_t)nkeys, -1);
+    int acc = 0;
+    for (long long k = 0; k < nkeys; k++) {
+        if (keycnt[k] == 0) continue;
+        keypos[k] = acc;
+        acc += keycnt[k];
+        pair_ab.push_back(make_int2((int)(k / nagg), (int)(k % nagg)));
+        pair_ptr.push_back(acc);
+    }
+    items.resize((size_t)h->nnzb);
+    for (int i = 0; i < N; i++)
+        for (int b = h->row_ptr_h[i]; b < h->row_ptr_h[i + 1]; b++)
+            items[(size_t)keypos[(size_t)aid[i] * nagg + aid[h->col_h[b]]]++] = make_int2(b, i);
 }
 
 // Plan of the one-launch PCG (pcg_resident.cu), made at the first solve that
@@ -1060,6 +1107,9 @@ int ensure_resident(SorsHandle* h) {
             for (int k = halo_ptr[b]; k < halo_ptr[b + 1]; k++) push[pos[halo[k]]++] = b << 16 | (k - halo_ptr[b]);
         for (int b = 0; b < pl.G; b++) pl.max_push = std::max(pl.max_push, push_ptr[row0[b + 1]] - push_ptr[row0[b]]);
     }
+    // the coarse correction, unless the settings rule it out: with one aggregate
+    // per range it costs no exchange of its own
+    pl.coarse = h->tl_req != 0 && pl.G >= 4 ? 1 : 0;
     const size_t fixed = resident_smem(pl, hs, 0);
     if (fixed > (size_t)kResidentSmem) return SORS_OK;
     pl.res_blocks = std::min(pl.max_over, (int)((kResidentSmem - fixed) / (9 * (size_t)hs)));
@@ -1068,7 +1118,7 @@ int ensure_resident(SorsHandle* h) {
     // one allocation: z, mailboxes and epoch (zeroed), then the plan's arrays
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t zb = pl.cluster ? 0 : up((size_t)N * (hs == 4 ? 4 : 6) * 8);
-    const size_t bb = pl.cluster ? 0 : up((size_t)pl.G * 6 * kResidentBoxEntries * 8);
+    const size_t bb = pl.cluster ? 0 : up((size_t)pl.G * kResidentBoxWords * 8);
     std::vector<int> ints;
     auto put = [&](const std::vector<int>& v) {
         const size_t at = ints.size();
@@ -1092,8 +1142,61 @@ int ensure_resident(SorsHandle* h) {
     pl.row0 = id + i_row0; pl.halo_ptr = id + i_hp; pl.halo = id + i_halo; pl.over = id + i_over;
     pl.push_ptr = id + i_pp; pl.push = id + i_push;
     pl.lcol = (const uint16_t*)(ibase + ib);
+    if (pl.coarse) {
+        // aggregate b: the nodes of range b; offsets from its centre, scaled by its mean extent
+        std::vector<double> X((size_t)h->ndof);
+        CK(d2h(h, X.data(), h->X, sizeof(double) * X.size()));
+        std::vector<float4> off(N);
+        for (int b = 0; b < pl.G; b++) {
+            const int a0 = row0[b], a1 = row0[b + 1], n = std::max(1, a1 - a0);
+            double c[3] = {0, 0, 0}, e2 = 0.0;
+            for (int i = a0; i < a1; i++)
+                for (int k = 0; k < 3; k++) c[k] += X[3 * (size_t)i + k] / n;
+            for (int i = a0; i < a1; i++)
+                for (int k = 0; k < 3; k++) e2 += (X[3 * (size_t)i + k] - c[k]) * (X[3 * (size_t)i + k] - c[k]) / n;
+            const double sc = e2 > 0.0 ? 1.0 / sqrt(e2) : 1.0;
+            for (int i = a0; i < a1; i++)
+                off[i] = make_float4((float)((X[3 * (size_t)i] - c[0]) * sc), (float)((X[3 * (size_t)i + 1] - c[1]) * sc),
+                                     (float)((X[3 * (size_t)i + 2] - c[2]) * sc), 0.0f);
+        }
+        std::vector<int> pair_ptr;
+        std::vector<int2> pair_ab, items;
+        coarse_pairs(h, owner, pl.G, pair_ptr, pair_ab, items);
+        const int nc = 6 * pl.G;
+        float4* off_d = nullptr;
+        if ((st = upload(h, &off_d, off.data(), off.size()))) return st;
+        if ((st = upload(h, &h->rc_pair_ptr, pair_ptr.data(), pair_ptr.size()))) return st;
+        if ((st = upload(h, &h->rc_ab, pair_ab.data(), pair_ab.size()))) return st;
+        if ((st = upload(h, &h->rc_items, items.data(), items.size()))) return st;
+        if ((st = dalloc_t(h, &h->rc_Ac, (size_t)nc * nc + nc + coarse_work(nc)))) return st;
+        if ((st = dalloc(h, &h->rc_Ainv, (size_t)nc * nc * hs))) return st;
+        h->rc_diag = h->rc_Ac + (size_t)nc * nc;
+        h->rc_work = h->rc_diag + nc;
+        h->rc_npairs = (int)pair_ab.size();
+        h->rcargs.N = N; h->rcargs.nagg = pl.G; h->rcargs.nc = nc;
+        h->rcargs.fixed = h->node_mask; h->rcargs.off = off_d;
+        pl.off = off_d;
+    }
     h->res = pl;
     h->res_state = 1;
+    return SORS_OK;
+}
+
+// The one-launch PCG's coarse inverse, from the Hessian in h->H.
+template <typename VT>
+int build_resident_coarse(SorsHandle* h) {
+    const int nc = h->rcargs.nc;
+    CK(cudaMemsetAsync(h->rc_Ac, 0, sizeof(double) * ((size_t)nc * nc + nc), h->stream));
+    if (sizeof(VT) == 4)
+        launch_coarse_galerkin_f(h->rc_npairs, h->rc_pair_ptr, h->rc_items, h->rc_ab, h->col, (const float*)h->H,
+                                 h->nnzb, h->rcargs, h->rc_Ac, h->rc_diag, h->stream);
+    else
+        launch_coarse_galerkin_d(h->rc_npairs, h->rc_pair_ptr, h->rc_items, h->rc_ab, h->col, (const double*)h->H,
+                                 h->nnzb, h->rcargs, h->rc_Ac, h->rc_diag, h->stream);
+    launch_coarse_invert(nc, h->rc_Ac, h->rc_diag, h->rc_work, h->stream);
+    launch_to_vt_perm<VT>(nc, h->rc_Ac, (VT*)h->rc_Ainv, h->stream);
+    h->rc_ready = true;
+    h->tl_refreshes++;
     return SORS_OK;
 }
 
@@ -1105,6 +1208,16 @@ int pcg_resident(SorsHandle* h, double eta, double abs_tol, const double* g, boo
     a.x = (VT*)h->x; a.p0 = (VT*)h->p0; a.p1 = (VT*)h->p1; a.zg = h->res_zg; a.box = h->res_box;
     a.eta2 = eta * eta; a.abs_tol2 = abs_tol * abs_tol; a.maxit = h->s.pcg_max_iter;
     a.pflag = h->proj_flag; a.pn = h->proj_n; a.epoch = h->res_epoch; a.sc = h->sc;
+    a.fixed = h->node_mask;
+    bool refreshed = false;
+    if (h->res.coarse) {
+        if (!h->rc_ready) {
+            int st = build_resident_coarse<VT>(h);
+            if (st) return st;
+            refreshed = true;
+        }
+        a.Ainv = (const VT*)h->rc_Ainv;
+    }
     *ran = launch_pcg_resident<VT>(h->res, a, h->stream) == 0;
     if (!*ran) {
         cudaGetLastError();
@@ -1114,15 +1227,15 @@ int pcg_resident(SorsHandle* h, double eta, double abs_tol, const double* g, boo
     CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     if (h->sc_host->status & kFlagTimeout) return fail(SORS_ERR_CUDA, "the PCG blocks did not meet within the limit");
+    if (h->res.coarse) coarse_rate_check(h, refreshed, &h->rc_ref_rate, &h->rc_ready);
     return SORS_OK;
 }
 
 template <typename HT, typename VT>
 int pcg_solve(SorsHandle* h, double eta, double abs_tol, int* iters, const double* g = nullptr) {
     static_assert(std::is_same<HT, VT>::value, "PCG vectors have the matrix's type");
-    const bool plain = h->batch.nmem <= 1 && !(h->s.two_level && h->cargs.nc > 0);
     bool ran = false;
-    if (plain) {
+    if (h->batch.nmem <= 1) {
         h->tl_active = false;
         int st = ensure_resident(h);
         if (st) return st;
@@ -1140,6 +1253,8 @@ int pcg_solve(SorsHandle* h, double eta, double abs_tol, int* iters, const doubl
     }
     launch_block_jacobi<HT, VT>(h->N, h->row_ptr, h->diag_slot, (const HT*)h->H, h->nnzb, (VT*)h->Minv, h->stream);
     if (h->batch.nmem > 1) return pcg_solve_members<HT, VT>(h, eta, abs_tol, iters, g);
+    int st2 = ensure_two_level(h);
+    if (st2) return st2;
     // the two-level preconditioner: with a constraint projection (SQP, adjoint)
     // the correction is projected too, so the preconditioner stays SPD on the
     // free subspace (the coarse matrix itself is built without the projection)
@@ -1174,7 +1289,7 @@ int pcg_solve(SorsHandle* h, double eta, double abs_tol, int* iters, const doubl
         if (st) return st;
     }
     // loose solves converge faster per decade and are not counted
-    coarse_rate_check(h, refreshed);
+    if (h->tl_active) coarse_rate_check(h, refreshed, &h->tl_ref_rate, &h->tl_ready);
     if (h->sc_host->breakdown && h->sc_host->it == 0 && !(h->s.project_spd == 2 && !h->proj_fallback))
         return fail(SORS_ERR_PCG_BREAKDOWN, "PCG breakdown: the Hessian is not positive definite");
     return SORS_OK;
@@ -1200,6 +1315,8 @@ int minres_solve(SorsHandle* h, double dt, double eta, double abs_tol, int* iter
             int st = dalloc(h, &h->mr_w[k], sizeof(VT) * 3 * (size_t)h->N);
             if (st) return st;
         }
+    int st2 = ensure_two_level(h);
+    if (st2) return st2;
     h->tl_active = h->s.two_level && h->cargs.nc > 0;
     bool refreshed = false;
     if (h->tl_active && (!h->tl_ready || !h->tl_proj)) {
@@ -1275,7 +1392,7 @@ int minres_solve(SorsHandle* h, double dt, double eta, double abs_tol, int* iter
     }
     if (h->sc_host->mr_bad)
         return fail(SORS_ERR_PCG_BREAKDOWN, "MINRES breakdown: the preconditioner is not positive definite");
-    coarse_rate_check(h, refreshed);
+    if (h->tl_active) coarse_rate_check(h, refreshed, &h->tl_ref_rate, &h->tl_ready);
     return SORS_OK;
 }
 
@@ -1734,29 +1851,9 @@ int setup_two_level(SorsHandle* h, const double* X) {
         off[i] = make_float4((float)((X[3 * i] - c.x) * c.w), (float)((X[3 * i + 1] - c.y) * c.w),
                              (float)((X[3 * i + 2] - c.z) * c.w), 0.0f);
     }
-    // aggregate pairs and their Hessian blocks (counting sort by pair key)
-    const long long nkeys = (long long)nagg * nagg;
-    std::vector<int> keycnt((size_t)nkeys + 1, 0);
-    const int64_t nnzb = h->nnzb;
-    for (int i = 0; i < N; i++)
-        for (int b = h->row_ptr_h[i]; b < h->row_ptr_h[i + 1]; b++) keycnt[(size_t)aid[i] * nagg + aid[h->col_h[b]] + 1]++;
-    std::vector<int> pair_ptr{0};
-    std::vector<int2> pair_ab;
-    std::vector<long long> keypos((size_t)nkeys, -1);
-    long long acc = 0;
-    for (long long k = 0; k < nkeys; k++) {
-        if (keycnt[k + 1] == 0) continue;
-        keypos[k] = acc;
-        acc += keycnt[k + 1];
-        pair_ab.push_back(make_int2((int)(k / nagg), (int)(k % nagg)));
-        pair_ptr.push_back((int)acc);
-    }
-    std::vector<int2> items((size_t)nnzb);
-    for (int i = 0; i < N; i++)
-        for (int b = h->row_ptr_h[i]; b < h->row_ptr_h[i + 1]; b++) {
-            const long long k = (long long)aid[i] * nagg + aid[h->col_h[b]];
-            items[(size_t)keypos[k]++] = make_int2(b, i);
-        }
+    std::vector<int> pair_ptr;
+    std::vector<int2> pair_ab, items;
+    coarse_pairs(h, aid, nagg, pair_ptr, pair_ab, items);
     int st;
     h->tl_npairs = (int)pair_ab.size();
     const int nc = 6 * nagg;
@@ -1776,8 +1873,8 @@ int setup_two_level(SorsHandle* h, const double* X) {
     h->tl_ld = (nc + w16 - 1) / w16 * w16;
     if ((st = dalloc_t(h, &h->tl_yc, (size_t)h->tl_ld))) return st;
     CK(dzero(h, h->tl_yc, sizeof(double) * (size_t)h->tl_ld));
-    if ((st = dalloc_t(h, &h->tl_rowk, (size_t)nc))) return st;
-    if ((st = dalloc_t(h, &h->tl_colk, (size_t)nc))) return st;
+    if ((st = dalloc_t(h, &h->tl_diag, (size_t)nc))) return st;
+    if ((st = dalloc_t(h, &h->tl_work, coarse_work(nc)))) return st;
     if ((st = dalloc(h, &h->tl_Ainv, (size_t)nc * h->tl_ld * hsize(h)))) return st;
     // contiguous aggregates (aid non-decreasing in node order): the runs of the
     // node-parallel restriction
@@ -2632,9 +2729,14 @@ int sors_create(const double* X, int32_t n_nodes, const int32_t* conn, int32_t n
     if ((st = upload(h, &h->node_mask, h->mask_h.data(), (size_t)N))) return bail(st);
     // two_level 2 ("auto"): on for meshes of 20,000 nodes or more, where the
     // coarse correction's three extra kernels per iteration pay for themselves
+    h->tl_req = h->s.two_level;
     if (h->s.two_level == 2) h->s.two_level = N >= 20000 ? 1 : 0;
-    if (h->s.two_level && (st = setup_two_level(h, X))) return bail(st);
     size_t hs = hsize(h);
+    // meshes the one-launch PCG may take (about 300 KB of matrix per SM) set it up at
+    // a solve that needs it
+    if (h->s.two_level && (size_t)h->nnzb * 9 * hs > ((size_t)kResidentMaxBlocks * 300 << 10) &&
+        (st = setup_two_level(h, X)))
+        return bail(st);
     // 160 bytes of padding: the SpMV reads values in 144-byte groups, the last of
     // which may run past the last block
     if ((st = dalloc(h, &h->H, (size_t)h->nnzb * 9 * hs + 160))) return bail(st);
@@ -2690,7 +2792,7 @@ int sors_set_neumann(SorsHandle* h, const int32_t* mask, const double* value) {
         CK(h2d(h, h->mval, vi.data(), sizeof(double) * h->ndof));
     }
     h->has_neumann = true;
-    h->tl_ready = false;  // the coarse space drops held DOFs
+    h->tl_ready = h->rc_ready = false;  // the coarse space drops held DOFs
     return SORS_OK;
 }
 
@@ -3477,6 +3579,7 @@ int profile_impl(SorsHandle* h, int iters, SorsKernelProfile* out) {
     out->pcg_update_ms = ms / iters;
     // p, q, Minv read; x, r read+written; z written
     out->pcg_update_bytes = 3 * N * vs * 2 + 9 * N * vs + 3 * N * vs * 4 + 3 * N * vs;
+    if ((st = ensure_two_level(h))) return st;
     if (h->cargs.nc > 0) {
         // two-level iteration kernels (their values are not used: timing only)
         CK(cudaMemsetAsync(&h->sc->done, 0, sizeof(int), h->stream));

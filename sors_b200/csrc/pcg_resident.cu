@@ -57,6 +57,7 @@ namespace {
 constexpr int kT = kResidentThreads;
 constexpr int kWarps = kT / 32;
 constexpr int kBoxes = kResidentBoxEntries;  // mailbox entries: five per polling lane
+constexpr int kScratch = 3328;
 constexpr int kPollLimit = 1 << 21;          // about a second
 static_assert(kResidentMaxBlocks <= kBoxes && kBoxes % 32 == 0, "a lane polls kBoxes / 32 entries");
 typedef unsigned long long u64;
@@ -70,18 +71,22 @@ struct Lay {
 
 // Byte offsets of a block's shared memory, the same in every block of a launch.
 struct Off {
-    int sp, sq, sm, sx, sz, sov, sgb, shalo, spp, spush, scol, sval;
+    int sp, sq, sm, sx, sz, soff, sa, syc, sov, sgb, shalo, spp, spush, scol, sval;
 };
 template <typename VT>
 __host__ __device__ inline Off offsets(const ResidentPlan& pl) {
     auto up = [](int b) { return (b + 15) & ~15; };
     Off o;
-    int at = 1024;  // Scratch
+    const int nc = pl.coarse ? 6 * pl.G : 0;
+    int at = kScratch;
     o.sp = at; at = up(at + pl.max_cols * Lay<VT>::P * (int)sizeof(VT));
     o.sq = at; at = up(at + pl.max_rows * 3 * (int)sizeof(VT));
     o.sm = at; at = up(at + pl.max_rows * 9 * (int)sizeof(VT));
     o.sx = at; at = up(at + pl.max_rows * 9 * (int)sizeof(VT));
     o.sz = at; at = up(at + (pl.cluster ? pl.max_halo * 4 * (int)sizeof(VT) : 0));
+    o.soff = at; at = up(at + (pl.coarse ? pl.max_rows * 16 : 0));
+    o.sa = at; at = up(at + 6 * nc * (int)sizeof(VT));
+    o.syc = at; at = up(at + 3 * nc * 8);
     o.sov = at; at = up(at + (pl.max_rows + 1) * 4);
     o.sgb = at; at = up(at + pl.max_rows * 4);
     o.shalo = at; at = up(at + (pl.cluster ? 0 : pl.max_halo * 4));
@@ -133,52 +138,93 @@ __device__ __forceinline__ void push(unsigned dst, unsigned bar, float a, float 
                  : "memory");
 }
 
+// Exchange sites and their values: 0 p.q (and P^T q, six values, with the coarse
+// correction), 1 r.z and r.r, 2 P^T r (six values, coarse correction).
+constexpr int kMsg = 7;
+__host__ __device__ constexpr int site_at(int site) { return site == 0 ? 0 : (site == 1 ? kMsg : kMsg + 2); }
+static_assert(2 * (kMsg + 2 + 6) * kBoxes == kResidentBoxWords, "words of a mailbox");
+
 // Fixed scratch at the start of the block's shared memory.
 struct Scratch {
-    u64 bar[2];             // cluster form: one mbarrier per reduction site
-    double part[kWarps][2];
+    u64 bar[4];                    // cluster form: one mbarrier per site
+    double part[kWarps][8];        // warps' partial values
     double tot[2];
+    double zc[6][2];               // the range's coarse correction, two partial sums each
     int abort, pad;
-    alignas(16) double slot[2][16][2];  // cluster form: the blocks' partial sums, by reduction site (16-byte pushes)
+    double slot[kMsg + 2 + 6][16];  // cluster form: the blocks' messages, by value
 };
-static_assert(sizeof(Scratch) <= 1024, "fixed scratch");
+static_assert(sizeof(Scratch) <= kScratch, "fixed scratch");
 
-// Sums v, already summed within each warp, over all blocks; every thread gets
-// the totals.  SITE 0: p.q, 1: r.z and r.r (and border z).  The sites alternate,
-// so a slot or mailbox entry is written again only after every block has read
-// it.  halo_bytes: border z the block receives with site 1 (cluster form).
-// False: something did not arrive within the poll limit.
-template <int SITE, bool CL>
-__device__ __forceinline__ bool all_sum(double (&v)[SITE + 1], Scratch* sh, int G, unsigned epoch, u64* box,
-                                        unsigned parity, int halo_bytes) {
-    constexpr int NS = SITE + 1;
+// Exchanges the NV values whose per-warp sums are in sh->part: warp v < NV adds
+// value v over the block's warps, sends it to every block, and collects all
+// blocks' values.  The first NSUM values are summed (every thread gets the
+// totals in v), the others are left per block: yq[(v - NSUM) G + b] in the grid
+// form, sh->slot[site_at(SITE) + v][b] in the cluster form.  No site is used twice
+// in a row, so a slot or mailbox entry is written again only after every block
+// has read it.
+// halo_bytes: border z the block receives with site 1 (cluster form).  False:
+// something did not arrive within the poll limit.
+template <int SITE, int NV, int NSUM, bool CL>
+__device__ __forceinline__ bool exchange(double (&v)[NSUM ? NSUM : 1], Scratch* sh, int G, unsigned epoch, u64* box,
+                                         unsigned parity, int halo_bytes, double* yq) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, me = blockIdx.x;
-    if (l == 0)
-#pragma unroll
-        for (int s = 0; s < NS; s++) sh->part[w][s] = v[s];
     __syncthreads();
-    if (w == 0) {
+    if (w < NV) {
+        double x = sh->part[l & (kWarps - 1)][w];
 #pragma unroll
-        for (int s = 0; s < NS; s++) v[s] = sh->part[l & (kWarps - 1)][s];
+        for (int o = kWarps / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if constexpr (CL) {
+            double* slot = sh->slot[site_at(SITE) + w];
+            if (w == 0 && l == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                                 (unsigned)__cvta_generic_to_shared(&sh->bar[SITE])),
+                             "r"(G * 8 * NV + halo_bytes)
+                             : "memory");
+            __syncwarp();
+            if (l < G) push(remote(slot + me, l), remote(&sh->bar[SITE], l), x);
+        } else {
+            constexpr int J = kBoxes / 32;
+            u64 lo, hi;
+            split(x, epoch, lo, hi);
+            constexpr int kVals = kMsg + 2 + 6;
+            const size_t at = (size_t)site_at(SITE) + w;  // this value's entries of a mailbox
 #pragma unroll
-        for (int o = kWarps / 2; o > 0; o >>= 1)
+            for (int j = 0; j < J; j++)
+                if (l + 32 * j < G)
+                    st_words(box + (((size_t)(l + 32 * j) * kVals + at) * kBoxes + me) * 2, lo, hi);
+            // a lane's entries are loaded together, so a round of polls is one trip to L2
+            const u64* q = box + (((size_t)me * kVals + at) * kBoxes + l) * 2;
+            u64 a[J], b[J];
+            bool ok;
+            int n = 0;
+            do {
+                ok = true;
 #pragma unroll
-            for (int s = 0; s < NS; s++) v[s] += __shfl_xor_sync(0xffffffffu, v[s], o);
+                for (int j = 0; j < J; j++)
+                    if (l + 32 * j < G) ld_words(q + 64 * j, a[j], b[j]);
+#pragma unroll
+                for (int j = 0; j < J; j++)
+                    if (l + 32 * j < G) ok = ok && has(a[j], epoch) && has(b[j], epoch);
+                ok = __all_sync(0xffffffffu, ok);  // the warp stays together
+            } while (!ok && ++n < kPollLimit);
+            if (w < NSUM) {
+                double t = 0.0;
+#pragma unroll
+                for (int j = 0; j < J; j++)
+                    if (l + 32 * j < G) t += join(a[j], b[j]);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (l == 0) sh->tot[w] = t;
+            } else {
+#pragma unroll
+                for (int j = 0; j < J; j++)
+                    if (l + 32 * j < G) yq[(w - NSUM) * G + l + 32 * j] = join(a[j], b[j]);
+            }
+            if (l == 0 && !ok) sh->abort = 1;
+        }
     }
     if constexpr (CL) {
         const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh->bar[SITE]);
-        if (w == 0) {
-            if (l == 0)
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                             "r"(G * 8 * NS + halo_bytes)
-                             : "memory");
-            __syncwarp();
-            if (l < G) {
-                const unsigned dst = remote(&sh->slot[SITE][me][0], l), rb = remote(&sh->bar[SITE], l);
-                if constexpr (NS == 1) push(dst, rb, v[0]);
-                else push(dst, rb, v[0], v[1]);
-            }
-        }
         unsigned got = 0;
         for (int n = 0; n < kPollLimit && !got; n++)
             asm volatile(
@@ -190,66 +236,16 @@ __device__ __forceinline__ bool all_sum(double (&v)[SITE + 1], Scratch* sh, int 
         if (!got) sh->abort = 1;
         // 16 values: a lane each (twice per warp), four shuffles
 #pragma unroll
-        for (int s = 0; s < NS; s++) v[s] = (l & 15) < G ? sh->slot[SITE][l & 15][s] : 0.0;
+        for (int s = 0; s < NSUM; s++) v[s] = (l & 15) < G ? sh->slot[site_at(SITE) + s][l & 15] : 0.0;
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
-            for (int s = 0; s < NS; s++) v[s] += __shfl_xor_sync(0xffffffffu, v[s], o);
+            for (int s = 0; s < NSUM; s++) v[s] += __shfl_xor_sync(0xffffffffu, v[s], o);
         return true;
     } else {
-        if (w == 0) {
-            constexpr int J = kBoxes / 32;
-            constexpr int kSite1 = 2 * kBoxes, kBox = 6 * kBoxes;  // words: site 0, then site 1
-            u64 lo[NS], hi[NS];
-#pragma unroll
-            for (int s = 0; s < NS; s++) split(v[s], epoch, lo[s], hi[s]);
-            const size_t at = SITE ? kSite1 : 0;
-#pragma unroll
-            for (int j = 0; j < J; j++)
-                if (l + 32 * j < G)
-#pragma unroll
-                    for (int s = 0; s < NS; s++)
-                        st_words(box + (size_t)(l + 32 * j) * kBox + at + (size_t)me * 2 * NS + 2 * s, lo[s], hi[s]);
-            // a lane's entries are loaded together, so a round of polls is one trip to L2
-            const u64* q = box + (size_t)me * kBox + at + (size_t)l * 2 * NS;
-            u64 a[J][NS], b[J][NS];
-            bool ok;
-            int n = 0;
-            do {
-                ok = true;
-#pragma unroll
-                for (int j = 0; j < J; j++)
-                    if (l + 32 * j < G)
-#pragma unroll
-                        for (int s = 0; s < NS; s++) ld_words(q + 64 * NS * j + 2 * s, a[j][s], b[j][s]);
-#pragma unroll
-                for (int j = 0; j < J; j++)
-                    if (l + 32 * j < G)
-#pragma unroll
-                        for (int s = 0; s < NS; s++) ok = ok && has(a[j][s], epoch) && has(b[j][s], epoch);
-                ok = __all_sync(0xffffffffu, ok);  // the warp stays together
-            } while (!ok && ++n < kPollLimit);
-            double t[NS];
-#pragma unroll
-            for (int s = 0; s < NS; s++) t[s] = 0.0;
-#pragma unroll
-            for (int j = 0; j < J; j++)
-                if (l + 32 * j < G)
-#pragma unroll
-                    for (int s = 0; s < NS; s++) t[s] += join(a[j][s], b[j][s]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int s = 0; s < NS; s++) t[s] += __shfl_xor_sync(0xffffffffu, t[s], o);
-            if (l == 0) {
-#pragma unroll
-                for (int s = 0; s < NS; s++) sh->tot[s] = t[s];
-                if (!ok) sh->abort = 1;
-            }
-        }
         __syncthreads();
 #pragma unroll
-        for (int s = 0; s < NS; s++) v[s] = sh->tot[s];
+        for (int s = 0; s < NSUM; s++) v[s] = sh->tot[s];
         return sh->abort == 0;
     }
 }
@@ -283,7 +279,25 @@ __device__ __forceinline__ void ld_p(const VT* p, VT& a, VT& b, VT& c) {
 __device__ __forceinline__ void keep(float& v) { asm volatile("" : "+f"(v)); }
 __device__ __forceinline__ void keep(double& v) { asm volatile("" : "+d"(v)); }
 
-template <typename VT, int LPR, int R, bool CL>
+// P_i^T y (six values) at a node with offset o from its range's centre: three
+// translations, three rotations; bits 0-2 of f: held DOFs.
+template <typename VT>
+__device__ __forceinline__ void restrict_node(const float4& o, unsigned f, const VT (&y)[3], double (&c)[6]) {
+    const double w0 = f & 1u ? 0.0 : (double)y[0], w1 = f & 2u ? 0.0 : (double)y[1], w2 = f & 4u ? 0.0 : (double)y[2];
+    const double dx = o.x, dy = o.y, dz = o.z;
+    c[0] += w0;
+    c[1] += w1;
+    c[2] += w2;
+    c[3] += dy * w2 - dz * w1;
+    c[4] += dz * w0 - dx * w2;
+    c[5] += dx * w1 - dy * w0;
+}
+
+// TL: the two-level preconditioner M^-1 + P Ac^-1 P^T with one aggregate per
+// range.  Every block keeps the whole y = P^T r (6 G values) and its own six
+// rows of Ac^-1: P^T q travels with p.q, y -= alpha P^T q is formed by every
+// block alike, and the correction costs no exchange of its own.
+template <typename VT, int LPR, int R, bool CL, bool TL>
 __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, ResidentArgs<VT> a) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int P = Lay<VT>::P, Z = Lay<VT>::Z;
@@ -301,6 +315,9 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
     int* spush = reinterpret_cast<int*>(smem + o.spush);
     uint16_t* scol = reinterpret_cast<uint16_t*>(smem + o.scol);
     VT* sval = reinterpret_cast<VT*>(smem + o.sval);
+    float4* soff = reinterpret_cast<float4*>(smem + o.soff);
+    VT* sa = reinterpret_cast<VT*>(smem + o.sa);
+    double* syc = reinterpret_cast<double*>(smem + o.syc);  // y, its next value, P^T q
     const int t = threadIdx.x, lane = t & 31, G = gridDim.x, me = blockIdx.x;
     const int r0 = pl.row0[me], nr = pl.row0[me + 1] - r0;
     const int h0 = pl.halo_ptr[me], nh = pl.halo_ptr[me + 1] - h0;
@@ -309,7 +326,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
         sh->abort = 0;
         if constexpr (CL)
 #pragma unroll
-            for (int k = 0; k < 2; k++)
+            for (int k = 0; k < 3; k++)
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&sh->bar[k]))
                              : "memory");
         if constexpr (CL) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -352,6 +369,18 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
         for (int k = t; k < nh; k += kT) shalo[k] = pl.halo[h0 + k];
     }
     for (int k = t; k < (nr + nh) * P; k += kT) sp[k] = VT(0);
+    const int nc = 6 * G;
+    if constexpr (TL) {
+        for (int k = t; k < 6 * nc; k += kT) sa[k] = __ldg(a.Ainv + (size_t)6 * me * nc + k);
+        for (int i = t; i < nr; i += kT) {
+            float4 v = pl.off[r0 + i];
+            v.w = __uint_as_float((unsigned)a.fixed[r0 + i] | (a.pflag ? (unsigned)a.pflag[r0 + i] << 8 : 0u));
+            soff[i] = v;
+        }
+    }
+    if (t < kWarps)
+#pragma unroll
+        for (int k = 0; k < 8; k++) sh->part[t][k] = 0.0;
 
     // one thread per row: x, r, z and the inverse diagonal block (as k_block_jacobi), in
     // shared memory (a row's nine values are an odd stride: no bank conflicts), so that
@@ -386,14 +415,25 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
     }
     __syncthreads();
 
-    // z = M^-1 r, published with the coming site-1 sum; r.z and r.r of the warp
-    auto precondition = [&](double (&acc)[2]) {
-        acc[0] = acc[1] = 0.0;
+    // z = M^-1 r (+ P zc), published with the coming site-1 sum; r.z and r.r of the warp
+    auto precondition = [&]() {
+        double acc[2] = {0.0, 0.0};
         if (t < nr) {
             VT z[3];
             const VT r[3] = {rs[0], rs[1], rs[2]};
 #pragma unroll
             for (int k = 0; k < 3; k++) z[k] = M[k * 3] * r[0] + M[k * 3 + 1] * r[1] + M[k * 3 + 2] * r[2];
+            if constexpr (TL) {
+                VT c[6];
+#pragma unroll
+                for (int m = 0; m < 6; m++) c[m] = (VT)(sh->zc[m][0] + sh->zc[m][1]);
+                const float4 d = soff[t];
+                const unsigned f = __float_as_uint(d.w);
+                const VT ox = (VT)d.x, oy = (VT)d.y, oz = (VT)d.z;
+                if (!(f & 1u)) z[0] += c[0] + c[4] * oz - c[5] * oy;
+                if (!(f & 2u)) z[1] += c[1] - c[3] * oz + c[5] * ox;
+                if (!(f & 4u)) z[2] += c[2] + c[3] * oy - c[4] * ox;
+            }
             project<VT>(pf, a.pn + row, z);
 #pragma unroll
             for (int k = 0; k < 3; k++) zs[k] = z[k];
@@ -434,12 +474,62 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
                 acc[1] += __shfl_xor_sync(0xffffffffu, acc[1], s);
             }
         }
+        if (lane == 0) {
+            sh->part[t >> 5][0] = acc[0];
+            sh->part[t >> 5][1] = acc[1];
+        }
+    };
+    // zc = Ac^-1 y for the range's six coarse unknowns, two warps a row, with
+    // y = ya - al P^T q (site 0's message), or the site-2 message itself (fresh); the
+    // first row's warps keep y in yb.
+    constexpr int kCW = 4;  // first of the twelve warps
+    auto coarse = [&](bool fresh, double al, const double* ya, double* yb) {
+        const int w = (t >> 5) - kCW;
+        if (w >= 0) {
+            const int m = w >> 1;
+            double z = 0.0;
+            for (int j = (w & 1) * 32 + lane; j < nc; j += 64) {
+                double y;
+                if constexpr (CL) y = sh->slot[site_at(fresh ? 2 : 0) + (fresh ? 0 : 1) + j / G][j % G];
+                else y = syc[2 * nc + j];
+                if (!fresh) y = ya[j] - al * y;
+                if (m == 0) yb[j] = y;
+                z += (double)sa[m * nc + j] * y;
+            }
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1) z += __shfl_xor_sync(0xffffffffu, z, s);
+            if (lane == 0) sh->zc[m][w & 1] = z;
+        }
+        __syncthreads();
+    };
+    unsigned par0 = 0, par1 = 0, par2 = 0;  // the sites' phases
+    int cur = 0;                            // which of the two y holds
+    // y = P^T r anew from the residual: at the start, and in FP32 every eighth
+    // iteration, so that y does not drift from the rounded r (y's own recurrence is FP64)
+    auto renew = [&]() {
+        double c[6] = {0, 0, 0, 0, 0, 0}, none[1];
+        if (t < nr) {
+            const VT r[3] = {rs[0], rs[1], rs[2]};
+            restrict_node<VT>(soff[t], __float_as_uint(soff[t].w), r, c);
+        }
+#pragma unroll
+        for (int m = 0; m < 6; m++) {
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1) c[m] += __shfl_xor_sync(0xffffffffu, c[m], s);
+            if (lane == 0) sh->part[t >> 5][m] = c[m];
+        }
+        const bool here = exchange<2, 6, 0, CL>(none, sh, G, ++epoch, a.box, par2, 0, syc + 2 * nc);
+        par2 ^= 1u;
+        coarse(true, 0.0, nullptr, syc + cur * nc);
+        return here;
     };
     constexpr int kZBytes = sizeof(VT) == 4 ? 16 : 24;
-    unsigned parity = 0;  // of both sites: they complete alternately, site 1 first
-    double acc[2];
-    precondition(acc);
-    bool ok = all_sum<1, CL>(acc, sh, G, ++epoch, a.box, 0u, nh * kZBytes);
+    bool ok = true;
+    double d1[1] = {0.0}, acc[2];
+    if constexpr (TL) ok = renew();
+    precondition();
+    ok = exchange<1, 2, 2, CL>(acc, sh, G, ++epoch, a.box, par1, nh * kZBytes, nullptr) && ok;
+    par1 ^= 1u;
     double rz = acc[0], rr = acc[1], pq = 0.0, alpha = 0.0, beta = 0.0;
     const double bnorm2 = rr;
     const double te = a.eta2 * rr, tol2 = te > a.abs_tol2 ? te : a.abs_tol2;
@@ -490,7 +580,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
         // and a warp in pieces runs what follows once per piece
         __syncwarp();
         __syncthreads();
-        double d1[1] = {0.0};
+        double pqw = 0.0, yw[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         for (int base = 0; base + (t & ~31) / LPR < nr; base += NG) {
             const int i = base + g;
             VT a0 = VT(0), a1 = VT(0), a2 = VT(0), p0, p1, p2;
@@ -529,13 +619,32 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
             if (i < nr) {
                 if (sl == 0) { sq[3 * i] = a0; sq[3 * i + 1] = a1; sq[3 * i + 2] = a2; }
                 ld_p<VT>(sp + P * i, p0, p1, p2);
-                d1[0] += (double)p0 * (double)a0 + (double)p1 * (double)a1 + (double)p2 * (double)a2;
+                pqw += (double)p0 * (double)a0 + (double)p1 * (double)a1 + (double)p2 * (double)a2;
+                if constexpr (TL) {
+                    const float4 d = soff[i];
+                    const unsigned f = __float_as_uint(d.w);
+                    VT q[3] = {a0, a1, a2};
+                    project<VT>(f >> 8, a.pn + r0 + i, q);
+                    restrict_node<VT>(d, f, q, yw);
+                }
             }
         }
-        // every lane of a group has its rows' share of p.q: add the warp's groups
+        // every lane of a group has its rows' share of the sums: add the warp's groups
 #pragma unroll
-        for (int s = 16; s >= LPR; s >>= 1) d1[0] += __shfl_xor_sync(0xffffffffu, d1[0], s);
-        ok = all_sum<0, CL>(d1, sh, G, ++epoch, a.box, parity, 0);
+        for (int s = 16; s >= LPR; s >>= 1) {
+            pqw += __shfl_xor_sync(0xffffffffu, pqw, s);
+            if constexpr (TL)
+#pragma unroll
+                for (int m = 0; m < 6; m++) yw[m] += __shfl_xor_sync(0xffffffffu, yw[m], s);
+        }
+        if (lane == 0) {
+            sh->part[t >> 5][0] = pqw;
+            if constexpr (TL)
+#pragma unroll
+                for (int m = 0; m < 6; m++) sh->part[t >> 5][1 + m] = yw[m];
+        }
+        ok = exchange<0, TL ? kMsg : 1, 1, CL>(d1, sh, G, ++epoch, a.box, par0, 0, syc + 2 * nc);
+        par0 ^= 1u;
         if (!ok) break;
         pq = d1[0];
         if (!(pq > 0.0)) {
@@ -555,9 +664,17 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
 #pragma unroll
             for (int k = 0; k < 3; k++) rs[k] -= al * q[k];
         }
-        precondition(acc);
-        parity ^= 1u;
-        ok = all_sum<1, CL>(acc, sh, G, ++epoch, a.box, parity, nh * kZBytes);
+        if constexpr (TL) {
+            if (sizeof(VT) == 4 && (it & 7) == 7) {
+                if (!renew()) break;
+            } else {
+                coarse(false, (double)al, syc + cur * nc, syc + (cur ^ 1) * nc);
+                cur ^= 1;
+            }
+        }
+        precondition();
+        ok = exchange<1, 2, 2, CL>(acc, sh, G, ++epoch, a.box, par1, nh * kZBytes, nullptr);
+        par1 ^= 1u;
         if (!ok) break;
         beta = acc[0] / rz;
         rz = acc[0];
@@ -588,9 +705,9 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
     }
 }
 
-template <typename VT, int LPR, int R, bool CL>
+template <typename VT, int LPR, int R, bool CL, bool TL>
 int launch_one(const ResidentPlan& pl, const ResidentArgs<VT>& a, cudaStream_t st) {
-    auto kern = k_pcg_resident<VT, LPR, R, CL>;
+    auto kern = k_pcg_resident<VT, LPR, R, CL, TL>;
     static std::atomic<int> done[kMaxDevices];
     int dev = 0;
     cudaGetDevice(&dev);
@@ -622,12 +739,13 @@ int launch_one(const ResidentPlan& pl, const ResidentArgs<VT>& a, cudaStream_t s
     return 0;
 }
 
-template <typename VT, bool CL>
+template <typename VT, bool CL, bool TL>
 int launch_shape(const ResidentPlan& pl, const ResidentArgs<VT>& a, cudaStream_t st) {
-    if (pl.lpr == 8) return pl.reg == 2 ? launch_one<VT, 8, 2, CL>(pl, a, st) : launch_one<VT, 8, 4, CL>(pl, a, st);
+    if (pl.lpr == 8)
+        return pl.reg == 2 ? launch_one<VT, 8, 2, CL, TL>(pl, a, st) : launch_one<VT, 8, 4, CL, TL>(pl, a, st);
     if constexpr (sizeof(VT) == 4)
-        if (pl.lpr == 2) return launch_one<VT, 2, 8, CL>(pl, a, st);
-    return launch_one<VT, 4, 4, CL>(pl, a, st);
+        if (pl.lpr == 2) return launch_one<VT, 2, 8, CL, TL>(pl, a, st);
+    return launch_one<VT, 4, 4, CL, TL>(pl, a, st);
 }
 
 }  // namespace
@@ -640,7 +758,9 @@ size_t resident_smem(const ResidentPlan& pl, int vsize, int res) {
 
 template <typename VT>
 int launch_pcg_resident(const ResidentPlan& pl, const ResidentArgs<VT>& a, cudaStream_t st) {
-    return pl.cluster ? launch_shape<VT, true>(pl, a, st) : launch_shape<VT, false>(pl, a, st);
+    if (a.Ainv)
+        return pl.cluster ? launch_shape<VT, true, true>(pl, a, st) : launch_shape<VT, false, true>(pl, a, st);
+    return pl.cluster ? launch_shape<VT, true, false>(pl, a, st) : launch_shape<VT, false, false>(pl, a, st);
 }
 template int launch_pcg_resident<float>(const ResidentPlan&, const ResidentArgs<float>&, cudaStream_t);
 template int launch_pcg_resident<double>(const ResidentPlan&, const ResidentArgs<double>&, cudaStream_t);

@@ -178,9 +178,11 @@ void launch_bpcg_iter(const BatchArgs& b, const int* row_ptr, const int* col, co
 constexpr int kResidentThreads = 512;
 constexpr int kResidentMaxBlocks = 148;
 constexpr int kResidentBoxEntries = 160;
+constexpr int kResidentBoxWords = 2 * 15 * kResidentBoxEntries;  // 7 + 2 + 6 values, two words an entry
 constexpr int kResidentSmem = 232448;  // 227 KB, the most a block may have
 struct ResidentPlan {
     int G = 0, cluster = 0;             // blocks; 1: one cluster, 0: a cooperative grid
+    int coarse = 0;                     // room for the coarse correction (one aggregate per block)
     int lpr = 8, reg = 2;               // lanes per row, matrix blocks per lane in registers
     int max_rows = 0, max_cols = 0, max_halo = 0, max_over = 0, max_push = 0;  // largest of any block
     int res_blocks = 0;                 // matrix blocks in shared memory, of those not in registers
@@ -192,6 +194,7 @@ struct ResidentPlan {
     const int* push_ptr = nullptr;      // N + 1, cluster: the blocks that read a row's z ...
     const int* push = nullptr;          // ... as block << 16 | its border column
     const uint16_t* lcol = nullptr;     // per CSR block: row of the range, or rows + border column
+    const float4* off = nullptr;        // N, coarse: scaled offset from the range's centre
 };
 template <typename VT>
 struct ResidentArgs {
@@ -205,8 +208,10 @@ struct ResidentArgs {
     int maxit = 0;
     const uint8_t* pflag = nullptr;     // constraint projection (null: none)
     const double4* pn = nullptr;
+    const VT* Ainv = nullptr;           // coarse inverse (null: block Jacobi alone), 6 G rows; column m G + b: unknown m of block b
+    const uint8_t* fixed = nullptr;     // Neumann bits per node
     unsigned long long* zg = nullptr;   // grid form: published z, 4 (FP32) or 6 (FP64) words per node
-    unsigned long long* box = nullptr;  // grid form: mailboxes, 6 x kResidentBoxEntries words per block
+    unsigned long long* box = nullptr;  // grid form: mailboxes, kResidentBoxWords per block
     unsigned* epoch = nullptr;          // grid form: the last epoch used
     DevScalars* sc = nullptr;
 };
@@ -232,13 +237,19 @@ struct CoarseArgs {
 };
 void launch_coarse_galerkin_f(int npairs, const int* cpair_ptr, const int2* cpair_items, const int2* cpair_ab,
                               const int* col, const float* H, long long nnzb, const CoarseArgs& c, double* Ac,
-                              cudaStream_t st);
+                              double* diag, cudaStream_t st);
 void launch_coarse_galerkin_d(int npairs, const int* cpair_ptr, const int2* cpair_items, const int2* cpair_ab,
                               const int* col, const double* H, long long nnzb, const CoarseArgs& c, double* Ac,
-                              cudaStream_t st);
-void launch_coarse_invert(int nc, double* Ac, double* rowk, double* colk, cudaStream_t st);
+                              double* diag, cudaStream_t st);
+// In-place inverse; diag: Ac's diagonal, work: coarse_work(nc) doubles.
+void launch_coarse_invert(int nc, double* Ac, const double* diag, double* work, cudaStream_t st);
+constexpr int kCoarsePanel = 32;
+inline size_t coarse_work(int nc) { return (size_t)2 * kCoarsePanel * nc + kCoarsePanel * kCoarsePanel; }
 template <typename VT>
 void launch_to_vt_pad(int nc, int ld, const double* in, VT* out, cudaStream_t st);
+// column 6 b + m of `in` as column m nagg + b of `out` (the one-launch PCG's order)
+template <typename VT>
+void launch_to_vt_perm(int nc, const double* in, VT* out, cudaStream_t st);
 template <typename VT>
 void launch_coarse_restrict(const CoarseArgs& c, const VT* r, double* yc, cudaStream_t st);
 template <typename VT>
