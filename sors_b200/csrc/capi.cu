@@ -214,8 +214,7 @@ struct SorsHandle {
     // its two-level preconditioner: one aggregate per row range
     CoarseArgs rcargs;
     int rc_npairs = 0;
-    int* rc_pair_ptr = nullptr;
-    int2 *rc_items = nullptr, *rc_ab = nullptr;
+    const int2* rc_ab = nullptr;
     double *rc_Ac = nullptr, *rc_diag = nullptr, *rc_work = nullptr;
     void* rc_Ainv = nullptr;
     bool rc_ready = false;
@@ -1115,38 +1114,15 @@ int ensure_resident(SorsHandle* h) {
     pl.res_blocks = std::min(pl.max_over, (int)((kResidentSmem - fixed) / (9 * (size_t)hs)));
     pl.smem_bytes = (int)resident_smem(pl, hs, pl.res_blocks);
     if (!pl.cluster && 2 * pl.res_blocks < pl.max_over) return SORS_OK;
-    // one allocation: z, mailboxes and epoch (zeroed), then the plan's arrays
-    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    const size_t zb = pl.cluster ? 0 : up((size_t)N * (hs == 4 ? 4 : 6) * 8);
-    const size_t bb = pl.cluster ? 0 : up((size_t)pl.G * kResidentBoxWords * 8);
-    std::vector<int> ints;
-    auto put = [&](const std::vector<int>& v) {
-        const size_t at = ints.size();
-        ints.insert(ints.end(), v.begin(), v.end());
-        return at;
-    };
-    const size_t i_row0 = put(row0), i_hp = put(halo_ptr), i_halo = put(halo), i_over = put(over),
-                 i_pp = put(push_ptr), i_push = put(push);
-    const size_t ib = up(ints.size() * sizeof(int));
-    char* base = nullptr;
-    int st;
-    if ((st = dalloc(h, (void**)&base, zb + bb + 256 + ib + lcol.size() * 2))) return st;
-    CK(cudaMemsetAsync(base, 0, zb + bb + 256, h->stream));
-    h->res_zg = (unsigned long long*)base;
-    h->res_box = (unsigned long long*)(base + zb);
-    h->res_epoch = (unsigned*)(base + zb + bb);
-    char* ibase = base + zb + bb + 256;
-    CK(h2d(h, ibase, ints.data(), ints.size() * sizeof(int)));
-    CK(h2d(h, ibase + ib, lcol.data(), lcol.size() * 2));
-    const int* id = (const int*)ibase;
-    pl.row0 = id + i_row0; pl.halo_ptr = id + i_hp; pl.halo = id + i_halo; pl.over = id + i_over;
-    pl.push_ptr = id + i_pp; pl.push = id + i_push;
-    pl.lcol = (const uint16_t*)(ibase + ib);
+    std::vector<float4> off;
+    std::vector<int2> ab;
+    const int nc = pl.coarse ? 6 * pl.G : 0;
     if (pl.coarse) {
         // aggregate b: the nodes of range b; offsets from its centre, scaled by its mean extent
         std::vector<double> X((size_t)h->ndof);
         CK(d2h(h, X.data(), h->X, sizeof(double) * X.size()));
-        std::vector<float4> off(N);
+        off.resize(N);
+        std::vector<int> met(pl.G, -1);
         for (int b = 0; b < pl.G; b++) {
             const int a0 = row0[b], a1 = row0[b + 1], n = std::max(1, a1 - a0);
             double c[3] = {0, 0, 0}, e2 = 0.0;
@@ -1158,25 +1134,52 @@ int ensure_resident(SorsHandle* h) {
             for (int i = a0; i < a1; i++)
                 off[i] = make_float4((float)((X[3 * (size_t)i] - c[0]) * sc), (float)((X[3 * (size_t)i + 1] - c[1]) * sc),
                                      (float)((X[3 * (size_t)i + 2] - c[2]) * sc), 0.0f);
+            // the ranges its blocks couple it to: its own and those of its border columns
+            if (a1 > a0) ab.push_back(make_int2(b, b));
+            for (int k = halo_ptr[b]; k < halo_ptr[b + 1]; k++) {
+                const int o = owner[halo[k]];
+                if (met[o] != b) ab.push_back(make_int2(b, o));
+                met[o] = b;
+            }
         }
-        std::vector<int> pair_ptr;
-        std::vector<int2> pair_ab, items;
-        coarse_pairs(h, owner, pl.G, pair_ptr, pair_ab, items);
-        const int nc = 6 * pl.G;
-        float4* off_d = nullptr;
-        if ((st = upload(h, &off_d, off.data(), off.size()))) return st;
-        if ((st = upload(h, &h->rc_pair_ptr, pair_ptr.data(), pair_ptr.size()))) return st;
-        if ((st = upload(h, &h->rc_ab, pair_ab.data(), pair_ab.size()))) return st;
-        if ((st = upload(h, &h->rc_items, items.data(), items.size()))) return st;
-        if ((st = dalloc_t(h, &h->rc_Ac, (size_t)nc * nc + nc + coarse_work(nc)))) return st;
-        if ((st = dalloc(h, &h->rc_Ainv, (size_t)nc * nc * hs))) return st;
-        h->rc_diag = h->rc_Ac + (size_t)nc * nc;
-        h->rc_work = h->rc_diag + nc;
-        h->rc_npairs = (int)pair_ab.size();
-        h->rcargs.N = N; h->rcargs.nagg = pl.G; h->rcargs.nc = nc;
-        h->rcargs.fixed = h->node_mask; h->rcargs.off = off_d;
-        pl.off = off_d;
     }
+    // one allocation: z, mailboxes and epoch (zeroed), the coarse matrices, then the
+    // plan's arrays in one copy
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    std::vector<char> host;
+    auto put = [&](const void* p, size_t bytes) {
+        const size_t at = host.size();
+        host.resize(at + up(bytes));
+        memcpy(host.data() + at, p, bytes);
+        return at;
+    };
+    auto puti = [&](const std::vector<int>& v) { return put(v.data(), v.size() * sizeof(int)); };
+    const size_t i_row0 = puti(row0), i_hp = puti(halo_ptr), i_halo = puti(halo), i_over = puti(over),
+                 i_pp = puti(push_ptr), i_push = puti(push), i_lcol = put(lcol.data(), lcol.size() * 2),
+                 i_off = put(off.data(), off.size() * sizeof(float4)), i_ab = put(ab.data(), ab.size() * sizeof(int2));
+    const size_t zb = pl.cluster ? 0 : up((size_t)N * (hs == 4 ? 4 : 6) * 8);
+    const size_t bb = pl.cluster ? 0 : up((size_t)pl.G * pl.G * kResidentBoxWords * 8);
+    const size_t cb = up(sizeof(double) * ((size_t)nc * nc + nc + coarse_work(nc))), vb = up((size_t)nc * nc * hs);
+    char* base = nullptr;
+    int st;
+    if ((st = dalloc(h, (void**)&base, zb + bb + 256 + cb + vb + host.size()))) return st;
+    CK(cudaMemsetAsync(base, 0, zb + bb + 256, h->stream));
+    h->res_zg = (unsigned long long*)base;
+    h->res_box = (unsigned long long*)(base + zb);
+    h->res_epoch = (unsigned*)(base + zb + bb);
+    h->rc_Ac = (double*)(base + zb + bb + 256);
+    h->rc_diag = h->rc_Ac + (size_t)nc * nc;
+    h->rc_work = h->rc_diag + nc;
+    h->rc_Ainv = base + zb + bb + 256 + cb;
+    char* d = (char*)h->rc_Ainv + vb;
+    CK(h2d(h, d, host.data(), host.size()));
+    pl.row0 = (const int*)(d + i_row0); pl.halo_ptr = (const int*)(d + i_hp); pl.halo = (const int*)(d + i_halo);
+    pl.over = (const int*)(d + i_over); pl.push_ptr = (const int*)(d + i_pp); pl.push = (const int*)(d + i_push);
+    pl.lcol = (const uint16_t*)(d + i_lcol); pl.off = (const float4*)(d + i_off);
+    h->rc_npairs = (int)ab.size();
+    h->rc_ab = (const int2*)(d + i_ab);
+    h->rcargs.N = N; h->rcargs.nagg = pl.G; h->rcargs.nc = nc;
+    h->rcargs.fixed = h->node_mask; h->rcargs.off = pl.off;
     h->res = pl;
     h->res_state = 1;
     return SORS_OK;
@@ -1187,12 +1190,8 @@ template <typename VT>
 int build_resident_coarse(SorsHandle* h) {
     const int nc = h->rcargs.nc;
     CK(cudaMemsetAsync(h->rc_Ac, 0, sizeof(double) * ((size_t)nc * nc + nc), h->stream));
-    if (sizeof(VT) == 4)
-        launch_coarse_galerkin_f(h->rc_npairs, h->rc_pair_ptr, h->rc_items, h->rc_ab, h->col, (const float*)h->H,
-                                 h->nnzb, h->rcargs, h->rc_Ac, h->rc_diag, h->stream);
-    else
-        launch_coarse_galerkin_d(h->rc_npairs, h->rc_pair_ptr, h->rc_items, h->rc_ab, h->col, (const double*)h->H,
-                                 h->nnzb, h->rcargs, h->rc_Ac, h->rc_diag, h->stream);
+    launch_range_galerkin<VT>(h->rc_npairs, h->rc_ab, h->res.row0, h->row_ptr, h->col, (const VT*)h->H, h->rcargs,
+                              h->rc_Ac, h->rc_diag, h->stream);
     launch_coarse_invert(nc, h->rc_Ac, h->rc_diag, h->rc_work, h->stream);
     launch_to_vt_perm<VT>(nc, h->rc_Ac, (VT*)h->rc_Ainv, h->stream);
     h->rc_ready = true;

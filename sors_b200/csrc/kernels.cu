@@ -2607,6 +2607,56 @@ __device__ __forceinline__ void coarse_restrict_node(const CoarseArgs& c, int i,
 // (10,000 blocks) took 7.6 ms of a first solve at 22,680 nodes and 10.9 ms at
 // 522,801; diag receives Ac's diagonal.
 constexpr int kGalThreads = 128;
+
+// acc += P_i^T hb P_j (row-major 6 x 6)
+template <typename HT>
+__device__ __forceinline__ void galerkin_add(const CoarseArgs& c, int i, int j, const HT* __restrict__ hb,
+                                             double (&acc)[36]) {
+    const unsigned fi = c.fixed ? c.fixed[i] : 0u, fj = c.fixed ? c.fixed[j] : 0u;
+    double T[3][6];  // hb P_j, rows of held DOFs zero
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) T[r][k] = ((fi >> r) | (fj >> k)) & 1u ? 0.0 : (double)hb[3 * r + k];
+    const float4 oj = c.off[j], oi = c.off[i];
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        T[r][3] = (double)oj.y * T[r][2] - (double)oj.z * T[r][1];
+        T[r][4] = (double)oj.z * T[r][0] - (double)oj.x * T[r][2];
+        T[r][5] = (double)oj.x * T[r][1] - (double)oj.y * T[r][0];
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+#pragma unroll
+        for (int r = 0; r < 3; r++) acc[6 * r + k] += T[r][k];
+        acc[18 + k] += (double)oi.y * T[2][k] - (double)oi.z * T[1][k];
+        acc[24 + k] += (double)oi.z * T[0][k] - (double)oi.x * T[2][k];
+        acc[30 + k] += (double)oi.x * T[1][k] - (double)oi.y * T[0][k];
+    }
+}
+
+// The block's sum of acc into the pair's 6 x 6 block of Ac.
+__device__ __forceinline__ void galerkin_store(const CoarseArgs& c, double (&acc)[36],
+                                               double (*sh)[36], int2 p, double* __restrict__ Ac,
+                                               double* __restrict__ diag) {
+    const int t = threadIdx.x, w = t >> 5, l = t & 31;
+#pragma unroll
+    for (int k = 0; k < 36; k++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+        if (l == 0) sh[w][k] = acc[k];
+    }
+    __syncthreads();
+    if (t < 36) {
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < kGalThreads / 32; k++) v += sh[k][t];
+        const int r = t / 6, m = t - 6 * (t / 6);
+        Ac[(size_t)(6 * p.x + r) * c.nc + 6 * p.y + m] = v;
+        if (p.x == p.y && r == m) diag[6 * p.x + r] = v;
+    }
+}
+
 template <typename HT>
 __global__ void __launch_bounds__(kGalThreads) k_coarse_galerkin(int npairs, const int* __restrict__ cpair_ptr,
                                                                  const int2* __restrict__ items,
@@ -2624,48 +2674,46 @@ __global__ void __launch_bounds__(kGalThreads) k_coarse_galerkin(int npairs, con
     const int i1 = cpair_ptr[pr + 1];
     for (int it = cpair_ptr[pr] + t; it < i1; it += kGalThreads) {
         const int2 bi = items[it];
-        const int i = bi.y, j = __ldg(col + bi.x);
-        const HT* hb = H + hval((size_t)bi.x, 0, (size_t)nnzb);
-        const unsigned fi = c.fixed ? c.fixed[i] : 0u, fj = c.fixed ? c.fixed[j] : 0u;
-        double T[3][6];  // H_ij P_j, rows of held DOFs zero
-#pragma unroll
-        for (int r = 0; r < 3; r++)
-#pragma unroll
-            for (int k = 0; k < 3; k++) T[r][k] = ((fi >> r) | (fj >> k)) & 1u ? 0.0 : (double)hb[3 * r + k];
-        const float4 oj = c.off[j], oi = c.off[i];
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            T[r][3] = (double)oj.y * T[r][2] - (double)oj.z * T[r][1];
-            T[r][4] = (double)oj.z * T[r][0] - (double)oj.x * T[r][2];
-            T[r][5] = (double)oj.x * T[r][1] - (double)oj.y * T[r][0];
-        }
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-#pragma unroll
-            for (int r = 0; r < 3; r++) acc[6 * r + k] += T[r][k];
-            acc[18 + k] += (double)oi.y * T[2][k] - (double)oi.z * T[1][k];
-            acc[24 + k] += (double)oi.z * T[0][k] - (double)oi.x * T[2][k];
-            acc[30 + k] += (double)oi.x * T[1][k] - (double)oi.y * T[0][k];
-        }
+        galerkin_add<HT>(c, bi.y, __ldg(col + bi.x), H + hval((size_t)bi.x, 0, (size_t)nnzb), acc);
     }
-    const int w = t >> 5, l = t & 31;
-#pragma unroll
-    for (int k = 0; k < 36; k++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-        if (l == 0) sh[w][k] = acc[k];
-    }
-    __syncthreads();
-    if (t < 36) {
-        double v = 0.0;
-#pragma unroll
-        for (int k = 0; k < kGalThreads / 32; k++) v += sh[k][t];
-        const int2 p = ab[pr];
-        const int r = t / 6, m = t - 6 * (t / 6);
-        Ac[(size_t)(6 * p.x + r) * c.nc + 6 * p.y + m] = v;
-        if (p.x == p.y && r == m) diag[6 * p.x + r] = v;
-    }
+    galerkin_store(c, acc, sh, ab[pr], Ac, diag);
 }
+
+// The same for aggregates that are row ranges: a thread walks rows of range a and
+// takes the blocks whose column lies in range b, so no item lists are made or
+// read (each row is read once per pair of its range, about 20 times, from L1 / L2).
+template <typename HT>
+__global__ void __launch_bounds__(kGalThreads) k_range_galerkin(const int2* __restrict__ ab,
+                                                                const int* __restrict__ row0,
+                                                                const int* __restrict__ row_ptr,
+                                                                const int* __restrict__ col,
+                                                                const HT* __restrict__ H, CoarseArgs c,
+                                                                double* __restrict__ Ac, double* __restrict__ diag) {
+    __shared__ double sh[kGalThreads / 32][36];
+    const int2 p = ab[blockIdx.x];
+    const int c0 = row0[p.y], c1 = row0[p.y + 1], i1 = row0[p.x + 1];
+    double acc[36];
+#pragma unroll
+    for (int k = 0; k < 36; k++) acc[k] = 0.0;
+    for (int i = row0[p.x] + threadIdx.x; i < i1; i += kGalThreads)
+        for (int b = __ldg(row_ptr + i); b < __ldg(row_ptr + i + 1); b++) {
+            const int j = __ldg(col + b);
+            if (j >= c0 && j < c1) galerkin_add<HT>(c, i, j, H + 9 * (size_t)b, acc);
+        }
+    galerkin_store(c, acc, sh, p, Ac, diag);
+}
+
+template <typename HT>
+void launch_range_galerkin(int npairs, const int2* ab, const int* row0, const int* row_ptr, const int* col,
+                           const HT* H, const CoarseArgs& c, double* Ac, double* diag, cudaStream_t st) {
+    if (npairs == 0) return;
+    k_range_galerkin<HT><<<npairs, kGalThreads, 0, st>>>(ab, row0, row_ptr, col, H, c, Ac, diag);
+    counted();
+}
+template void launch_range_galerkin<float>(int, const int2*, const int*, const int*, const int*, const float*,
+                                           const CoarseArgs&, double*, double*, cudaStream_t);
+template void launch_range_galerkin<double>(int, const int2*, const int*, const int*, const int*, const double*,
+                                            const CoarseArgs&, double*, double*, cudaStream_t);
 
 void launch_coarse_galerkin_f(int npairs, const int* cpair_ptr, const int2* cpair_items, const int2* cpair_ab,
                               const int* col, const float* H, long long nnzb, const CoarseArgs& c, double* Ac,

@@ -142,7 +142,8 @@ __device__ __forceinline__ void push(unsigned dst, unsigned bar, float a, float 
 // correction), 1 r.z and r.r, 2 P^T r (six values, coarse correction).
 constexpr int kMsg = 7;
 __host__ __device__ constexpr int site_at(int site) { return site == 0 ? 0 : (site == 1 ? kMsg : kMsg + 2); }
-static_assert(2 * (kMsg + 2 + 6) * kBoxes == kResidentBoxWords, "words of a mailbox");
+constexpr int kVals = kMsg + 2 + 6;
+static_assert(2 * kVals == kResidentBoxWords, "words of a mailbox entry");
 
 // Fixed scratch at the start of the block's shared memory.
 struct Scratch {
@@ -151,7 +152,7 @@ struct Scratch {
     double tot[2];
     double zc[6][2];               // the range's coarse correction, two partial sums each
     int abort, pad;
-    double slot[kMsg + 2 + 6][16];  // cluster form: the blocks' messages, by value
+    double slot[kVals][16];  // cluster form: the blocks' messages, by value
 };
 static_assert(sizeof(Scratch) <= kScratch, "fixed scratch");
 
@@ -186,14 +187,13 @@ __device__ __forceinline__ bool exchange(double (&v)[NSUM ? NSUM : 1], Scratch* 
             constexpr int J = kBoxes / 32;
             u64 lo, hi;
             split(x, epoch, lo, hi);
-            constexpr int kVals = kMsg + 2 + 6;
             const size_t at = (size_t)site_at(SITE) + w;  // this value's entries of a mailbox
 #pragma unroll
             for (int j = 0; j < J; j++)
                 if (l + 32 * j < G)
-                    st_words(box + (((size_t)(l + 32 * j) * kVals + at) * kBoxes + me) * 2, lo, hi);
+                    st_words(box + (((size_t)(l + 32 * j) * kVals + at) * G + me) * 2, lo, hi);
             // a lane's entries are loaded together, so a round of polls is one trip to L2
-            const u64* q = box + (((size_t)me * kVals + at) * kBoxes + l) * 2;
+            const u64* q = box + (((size_t)me * kVals + at) * G + l) * 2;
             u64 a[J], b[J];
             bool ok;
             int n = 0;

@@ -178,7 +178,7 @@ void launch_bpcg_iter(const BatchArgs& b, const int* row_ptr, const int* col, co
 constexpr int kResidentThreads = 512;
 constexpr int kResidentMaxBlocks = 148;
 constexpr int kResidentBoxEntries = 160;
-constexpr int kResidentBoxWords = 2 * 15 * kResidentBoxEntries;  // 7 + 2 + 6 values, two words an entry
+constexpr int kResidentBoxWords = 2 * 15;  // of a mailbox per sending block: 7 + 2 + 6 values, two words each
 constexpr int kResidentSmem = 232448;  // 227 KB, the most a block may have
 struct ResidentPlan {
     int G = 0, cluster = 0;             // blocks; 1: one cluster, 0: a cooperative grid
@@ -211,7 +211,7 @@ struct ResidentArgs {
     const VT* Ainv = nullptr;           // coarse inverse (null: block Jacobi alone), 6 G rows; column m G + b: unknown m of block b
     const uint8_t* fixed = nullptr;     // Neumann bits per node
     unsigned long long* zg = nullptr;   // grid form: published z, 4 (FP32) or 6 (FP64) words per node
-    unsigned long long* box = nullptr;  // grid form: mailboxes, kResidentBoxWords per block
+    unsigned long long* box = nullptr;  // grid form: mailboxes, G kResidentBoxWords per block
     unsigned* epoch = nullptr;          // grid form: the last epoch used
     DevScalars* sc = nullptr;
 };
@@ -241,6 +241,10 @@ void launch_coarse_galerkin_f(int npairs, const int* cpair_ptr, const int2* cpai
 void launch_coarse_galerkin_d(int npairs, const int* cpair_ptr, const int2* cpair_items, const int2* cpair_ab,
                               const int* col, const double* H, long long nnzb, const CoarseArgs& c, double* Ac,
                               double* diag, cudaStream_t st);
+// The same sums for aggregates that are the row ranges [row0[a], row0[a + 1]).
+template <typename HT>
+void launch_range_galerkin(int npairs, const int2* ab, const int* row0, const int* row_ptr, const int* col,
+                           const HT* H, const CoarseArgs& c, double* Ac, double* diag, cudaStream_t st);
 // In-place inverse; diag: Ac's diagonal, work: coarse_work(nc) doubles.
 void launch_coarse_invert(int nc, double* Ac, const double* diag, double* work, cudaStream_t st);
 constexpr int kCoarsePanel = 32;
