@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <new>
+#include <functional>
 #include <string>
 #include <thread>
 #include <limits>
@@ -206,6 +207,11 @@ struct SorsHandle {
     int64_t n_hess_evals = 0, n_grad_evals = 0;  // system evaluations with / without the Hessian
     bool graph_failed = false;
 
+    // row ranges of the one-launch PCGs (choose_parts, number_by_parts): parts_A
+    // consecutive parts per range, part k the nodes [part0[k], part0[k + 1]); empty part0:
+    // the numbering was not made by parts
+    int parts_form = 0, parts_G = 0, parts_A = 1;
+    std::vector<int> part0;
     // one-launch PCG (ensure_resident): 0 not looked at, 1 planned, -1 not for this mesh
     int res_state = 0;
     ResidentPlan res;
@@ -215,6 +221,15 @@ struct SorsHandle {
     CoarseArgs rcargs;
     int rc_npairs = 0;
     const int2* rc_ab = nullptr;
+    const int* rc_row0 = nullptr;       // first row of each aggregate
+    int rc_ld = 0;                      // leading dimension of rc_Ainv
+    // one-launch PCG with a streamed matrix (ensure_stream), for larger meshes: 0 not
+    // looked at, 1 planned, -1 not for this mesh
+    int str_state = 0;
+    StreamPlan str;
+    void* str_ws = nullptr;
+    float4* str_woff = nullptr;
+    unsigned long long* str_board = nullptr;
     double *rc_Ac = nullptr, *rc_diag = nullptr, *rc_work = nullptr;
     void* rc_Ainv = nullptr;
     bool rc_ready = false;
@@ -1015,6 +1030,77 @@ void coarse_pairs(const SorsHandle* h, const std::vector<int>& aid, int nagg, st
             items[(size_t)keypos[(size_t)aid[i] * nagg + aid[h->col_h[b]]]++] = make_int2(b, i);
 }
 
+// The form of the one-launch PCG and its number of row ranges, from the mesh's
+// size (before the pattern is built: tets have about 3 N + 2 E blocks, hexes N + 26 E):
+// 1 one cluster, 2 a grid with the matrix on the SMs, 3 a grid with a streamed matrix.
+void choose_parts(SorsHandle* h) {
+    const int N = h->N;
+    const size_t hs = hsize(h);
+    const double blocks = h->nv == 4 ? 3.0 * N + 2.0 * h->E : N + 26.0 * h->E, bytes = blocks * 9 * hs;
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) sms = 0;
+    // a handle whose grids are capped takes the same share of the SMs
+    int gmax = std::min(sms, kResidentMaxBlocks);
+    if (h->s.max_blocks > 0) gmax = std::min(gmax, std::max(1, h->s.max_blocks * kResidentMaxBlocks / kRedBlocks));
+    if (gmax < 1) return;
+    // One cluster up to 3.3 MB of matrix: its exchanges are three times cheaper,
+    // but 16 SMs hold and multiply the whole matrix.  Measured per iteration
+    // (cluster / grid): FP32 tets 2,744 nodes 3.7 / 5.3 us, 6,859 nodes (3.5 MB)
+    // 5.8 / 6.2 us; FP64 tets 1,000 nodes 4.0 / 6.2 us, 3,375 nodes (3.4 MB) 6.3 /
+    // 6.5 us, 4,225 nodes 7.6 / 6.5 us; FP64 hexes 891 nodes 13.6 / 18.1 us per
+    // adjoint iteration, 2,025 nodes 18.2 / 19.4 us.
+    h->parts_A = 1;
+    if (N <= 16 * kResidentThreads && bytes <= 16 * 200 * 1024.0) {
+        h->parts_form = 1;
+        h->parts_G = std::max(1, std::min(16, (N + 31) / 32));
+        return;
+    }
+    // Grid: 64 blocks, more where a block's rows would not have a lane group each.
+    // A sum over 148 blocks takes 2.2 us, over 64 1.4 us; 4,225 FP64 nodes per
+    // step: 148 blocks 5.6 ms, 96 5.0, 64 5.1, 36 5.4; 10,648 FP32 nodes per three
+    // steps: 148 blocks 48 ms, 96 44, 64 41, 36 50.
+    const int per = hs == 4 ? 160 : 128;
+    const int G = std::max(1, std::min({gmax, (N + 15) / 16, std::max(64, (N + per - 1) / per)}));
+    if (N <= G * (kResidentThreads - 16) && bytes <= G * 300 * 1024.0) {
+        h->parts_form = 2;
+        h->parts_G = G;
+        return;
+    }
+    if (h->s.max_blocks > 0 || !h->s.two_level) return;
+    // Streamed: while the ranges' p, with their border columns, and the rings fit in
+    // shared memory, and up to 2,500 rows a range (ms per step, launch per kernel /
+    // streamed: 77,841 FP32 nodes 11.2 / 6.7, 169,781 17.5 / 12.9, FP64 24.1 / 16.5,
+    // 291,870 25.3 / 19.8, 522,801 36.7 / 37.1).
+    const double rows = (double)N / gmax, border = 7.0 * pow(rows, 2.0 / 3.0);
+    const double ring = 16.0 * 8.0 * (h->nv == 4 ? 16.0 : 27.0) * (9.0 * hs + 2.0);
+    if (rows > 2500.0 ||
+        (rows + border) * (hs == 4 ? 16.0 : 24.0) + 4.0 * rows + 4.0 * border + 24e3 + ring > kResidentSmem)
+        return;
+    h->parts_form = 3;
+    h->parts_G = gmax;
+    // Aggregates per range: a second one takes a fifth off the iterations and adds
+    // the matrix of four times the coarse unknowns to each (ms per step, 1 / 2 / 4:
+    // 77,841 FP32 nodes 7.1 / 6.7 / 8.6, 169,781 14.2 / 12.9 / 14.2; 24,518: 4.3 / 4.5).
+    h->parts_A = rows < 400.0 ? 1 : 2;
+}
+
+// Rows of each of a range's A aggregates (the last may have fewer): whole warps.
+int part_rows(int n, int A) { return std::max(32, ((n + A - 1) / A + 31) / 32 * 32); }
+
+// First rows of G ranges: the numbering's parts (A per range), or ranges of about
+// equal numbers of matrix blocks.
+std::vector<int> range_rows(const SorsHandle* h, int G, int A) {
+    std::vector<int> row0(G + 1, 0);
+    row0[G] = h->N;
+    const std::vector<int>& rp = h->row_ptr_h;
+    for (int b = 1; b < G; b++)
+        row0[b] = (int)h->part0.size() == G * A + 1
+                      ? h->part0[(size_t)b * A]
+                      : std::max(row0[b - 1], (int)(std::lower_bound(rp.begin(), rp.end(), (int)(h->nnzb * b / G)) -
+                                                    rp.begin()));
+    return row0;
+}
+
 // Plan of the one-launch PCG (pcg_resident.cu), made at the first solve that
 // could use it: the row ranges, their border columns and local column indices.
 int ensure_resident(SorsHandle* h) {
@@ -1022,33 +1108,11 @@ int ensure_resident(SorsHandle* h) {
     h->res_state = -1;
     const int N = h->N;
     const int hs = (int)hsize(h);
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) return SORS_OK;
-    // a handle whose grids are capped takes the same share of the SMs
-    int gmax = std::min(sms, kResidentMaxBlocks);
-    if (h->s.max_blocks > 0) gmax = std::min(gmax, std::max(1, h->s.max_blocks * kResidentMaxBlocks / kRedBlocks));
-    const size_t bytes = (size_t)h->nnzb * 9 * hs;
     ResidentPlan pl;
-    // One cluster up to 3.3 MB of matrix: its exchanges are three times cheaper,
-    // but 16 SMs hold and multiply the whole matrix.  Measured per iteration
-    // (cluster / grid): FP32 tets 2,744 nodes 3.7 / 5.3 us, 6,859 nodes (3.5 MB)
-    // 5.8 / 6.2 us; FP64 tets 1,000 nodes 4.0 / 6.2 us, 3,375 nodes (3.4 MB) 6.3 /
-    // 6.5 us, 4,225 nodes 7.6 / 6.5 us; FP64 hexes 891 nodes 13.6 / 18.1 us per
-    // adjoint iteration, 2,025 nodes 18.2 / 19.4 us.
-    pl.cluster = (N <= 16 * kResidentThreads && bytes <= ((size_t)16 * 200 << 10)) ? 1 : 0;
-    // Grid: 64 blocks, more where a block's rows would not have a lane group each.
-    // A sum over 148 blocks takes 2.2 us, over 64 1.4 us; 4,225 FP64 nodes per
-    // step: 148 blocks 5.6 ms, 96 5.0, 64 5.1, 36 5.4; 10,648 FP32 nodes per three
-    // steps: 148 blocks 48 ms, 96 44, 64 41, 36 50.
-    const int per = hs == 4 ? 160 : 128;
-    pl.G = pl.cluster ? std::max(1, std::min(16, (N + 31) / 32))
-                      : std::max(1, std::min({gmax, (N + 15) / 16, std::max(64, (N + per - 1) / per)}));
-    // ranges of about equal numbers of matrix blocks
-    std::vector<int> row0(pl.G + 1, 0);
-    row0[pl.G] = N;
-    for (int b = 1; b < pl.G; b++)
-        row0[b] = std::max(row0[b - 1], (int)(std::lower_bound(h->row_ptr_h.begin(), h->row_ptr_h.end(),
-                                              (int)(h->nnzb * b / pl.G)) - h->row_ptr_h.begin()));
+    if (h->parts_form != 1 && h->parts_form != 2) return SORS_OK;
+    pl.cluster = h->parts_form == 1;
+    pl.G = h->parts_G;
+    const std::vector<int> row0 = range_rows(h, pl.G, 1);
     std::vector<int> owner(N), halo, halo_ptr(pl.G + 1, 0);
     for (int b = 0; b < pl.G; b++) {
         pl.max_rows = std::max(pl.max_rows, row0[b + 1] - row0[b]);
@@ -1178,10 +1242,171 @@ int ensure_resident(SorsHandle* h) {
     pl.lcol = (const uint16_t*)(d + i_lcol); pl.off = (const float4*)(d + i_off);
     h->rc_npairs = (int)ab.size();
     h->rc_ab = (const int2*)(d + i_ab);
+    h->rc_row0 = pl.row0;
+    h->rc_ld = nc;
     h->rcargs.N = N; h->rcargs.nagg = pl.G; h->rcargs.nc = nc;
     h->rcargs.fixed = h->node_mask; h->rcargs.off = pl.off;
     h->res = pl;
     h->res_state = 1;
+    return SORS_OK;
+}
+
+// Plan of the one-launch PCG with a streamed matrix (pcg_stream.cu), made at the
+// first solve of a mesh the resident form does not take.
+int ensure_stream(SorsHandle* h) {
+    if (h->str_state != 0) return SORS_OK;
+    h->str_state = -1;
+    const int N = h->N;
+    const int hs = (int)hsize(h);
+    if (h->parts_form != 3) return SORS_OK;
+    StreamPlan pl;
+    pl.G = h->parts_G;
+    pl.A = h->parts_A;
+    pl.N = N;
+    const int gr = 32 / pl.lpr;
+    const int nagg = pl.A * pl.G, G = pl.G;
+    pl.nc = 6 * nagg;
+    const int w16 = 16 / hs;
+    pl.ld = (pl.nc + w16 - 1) / w16 * w16;
+    const std::vector<int>& rp = h->row_ptr_h;
+    const std::vector<int> row0 = range_rows(h, G, pl.A);
+    std::vector<int> agg_rows(G), agg0(nagg + 1, N), aid(N);
+    size_t gbytes = 0, cbytes = 0;
+    for (int b = 0; b < G; b++) {
+        const int n = row0[b + 1] - row0[b];
+        pl.max_rows = std::max(pl.max_rows, n);
+        agg_rows[b] = part_rows(n, pl.A);
+        for (int k = 0; k < pl.A; k++) {
+            agg0[b * pl.A + k] = row0[b] + std::min(n, k * agg_rows[b]);
+            const int e = row0[b] + std::min(n, (k + 1) * agg_rows[b]);
+            for (int i = agg0[b * pl.A + k]; i < e; i++) aid[i] = b * pl.A + k;
+        }
+        for (int i = row0[b]; i < row0[b + 1]; i += gr) {
+            const size_t f0 = (size_t)rp[i] * 9 * hs & ~(size_t)15,
+                         f1 = ((size_t)rp[std::min(i + gr, row0[b + 1])] * 9 * hs + 15) & ~(size_t)15;
+            gbytes = std::max(gbytes, f1 - f0);
+            cbytes = std::max(cbytes, (((size_t)rp[std::min(i + gr, row0[b + 1])] * 2 + 15) & ~(size_t)15) -
+                                          ((size_t)rp[i] * 2 & ~(size_t)15));
+        }
+    }
+    pl.slot_col = (int)gbytes;
+    pl.slot_off = (int)(gbytes + cbytes);
+    pl.group_bytes = (int)(gbytes + cbytes) + 16 * gr;
+    // border columns and local column indices, the ranges over a few threads
+    std::vector<uint16_t> lcol((size_t)h->nnzb + 8);  // the last bulk copy rounds up to 16 bytes
+    std::vector<std::vector<int>> halos(G);
+    std::vector<std::vector<int2>> abs_(G);
+    const int nt = (int)std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
+    std::vector<std::thread> ts;
+    for (int k = 0; k < nt; k++)
+        ts.emplace_back([&, k]() {
+            std::vector<int> seen(N, -1), local(N), met(nagg, -1);
+            for (int b = k; b < G; b += nt) {
+                const int a0 = row0[b], a1 = row0[b + 1];
+                std::vector<int>& hl = halos[b];
+                for (int i = a0; i < a1; i++)
+                    for (int c = rp[i]; c < rp[i + 1]; c++) {
+                        const int j = h->col_h[c];
+                        if (met[aid[j]] != aid[i]) {
+                            met[aid[j]] = aid[i];
+                            abs_[b].push_back(make_int2(aid[i], aid[j]));
+                        }
+                        if (j >= a0 && j < a1) {
+                            lcol[c] = (uint16_t)(j - a0);
+                            continue;
+                        }
+                        if (seen[j] != b) {
+                            seen[j] = b;
+                            local[j] = (int)hl.size() + a1 - a0;
+                            hl.push_back(j);
+                        }
+                        lcol[c] = (uint16_t)local[j];
+                    }
+            }
+        });
+    for (auto& t : ts) t.join();
+    std::vector<int> halo_ptr(G + 1, 0), halo;
+    std::vector<uint8_t> border(N, 0);
+    std::vector<int2> ab;
+    for (int b = 0; b < G; b++) {
+        pl.max_cols = std::max(pl.max_cols, row0[b + 1] - row0[b] + (int)halos[b].size());
+        pl.max_halo = std::max(pl.max_halo, (int)halos[b].size());
+        for (int j : halos[b]) border[j] = 1;
+        halo.insert(halo.end(), halos[b].begin(), halos[b].end());
+        halo_ptr[b + 1] = (int)halo.size();
+        ab.insert(ab.end(), abs_[b].begin(), abs_[b].end());
+    }
+    if (pl.max_cols > 65535) return SORS_OK;
+    pl.evict_first = (size_t)h->nnzb * 9 * hs > ((size_t)90 << 20) ? 1 : 0;
+    pl.depth = 1;
+    pl.a_shared = 1;
+    if (stream_smem(pl, hs) > (size_t)kResidentSmem) pl.a_shared = 0;
+    if (stream_smem(pl, hs) > (size_t)kResidentSmem) return SORS_OK;
+    while (pl.depth < 4) {
+        pl.depth++;
+        if (stream_smem(pl, hs) > (size_t)kResidentSmem) { pl.depth--; break; }
+    }
+    std::vector<float4> off(N);
+    {
+        std::vector<double> X((size_t)h->ndof);
+        CK(d2h(h, X.data(), h->X, sizeof(double) * X.size()));
+        for (int k = 0; k < nagg; k++) {
+            const int a0 = agg0[k], a1 = agg0[k + 1], n = std::max(1, a1 - a0);
+            double c[3] = {0, 0, 0}, e2 = 0.0;
+            for (int i = a0; i < a1; i++)
+                for (int m = 0; m < 3; m++) c[m] += X[3 * (size_t)i + m] / n;
+            for (int i = a0; i < a1; i++)
+                for (int m = 0; m < 3; m++) e2 += (X[3 * (size_t)i + m] - c[m]) * (X[3 * (size_t)i + m] - c[m]) / n;
+            const double sc = e2 > 0.0 ? 1.0 / sqrt(e2) : 1.0;
+            for (int i = a0; i < a1; i++)
+                off[i] = make_float4((float)((X[3 * (size_t)i] - c[0]) * sc), (float)((X[3 * (size_t)i + 1] - c[1]) * sc),
+                                     (float)((X[3 * (size_t)i + 2] - c[2]) * sc), 0.0f);
+        }
+    }
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    std::vector<char> host;
+    auto put = [&](const void* p, size_t bytes) {
+        const size_t at = host.size();
+        host.resize(at + up(bytes));
+        memcpy(host.data() + at, p, bytes);
+        return at;
+    };
+    auto puti = [&](const std::vector<int>& v) { return put(v.data(), v.size() * sizeof(int)); };
+    const size_t i_row0 = puti(row0), i_hp = puti(halo_ptr), i_halo = puti(halo), i_ar = puti(agg_rows),
+                 i_agg0 = puti(agg0), i_ab = put(ab.data(), ab.size() * sizeof(int2)),
+                 i_off = put(off.data(), off.size() * sizeof(float4)), i_bd = put(border.data(), border.size()),
+                 i_lcol = put(lcol.data(), lcol.size() * 2);
+    const size_t nc = pl.nc;
+    const size_t zb = up((size_t)N * (hs == 4 ? 4 : 6) * 8), bb = up((size_t)G * G * kResidentBoxWords * 8),
+                 ob = up(3 * 2 * nc * 8), wb = up((size_t)18 * N * hs), fb = up((size_t)N * sizeof(float4)),
+                 cb = up(sizeof(double) * (nc * nc + nc + coarse_work((int)nc))), vb = up(nc * pl.ld * hs);
+    char* base = nullptr;
+    int st;
+    if ((st = dalloc(h, (void**)&base, zb + bb + ob + 256 + wb + fb + cb + vb + host.size()))) return st;
+    CK(cudaMemsetAsync(base, 0, zb + bb + ob + 256, h->stream));
+    char* q = base;
+    h->res_zg = (unsigned long long*)q; q += zb;
+    h->res_box = (unsigned long long*)q; q += bb;
+    h->str_board = (unsigned long long*)q; q += ob;
+    h->res_epoch = (unsigned*)q; q += 256;
+    h->str_ws = q; q += wb;
+    h->str_woff = (float4*)q; q += fb;
+    h->rc_Ac = (double*)q; q += cb;
+    h->rc_diag = h->rc_Ac + nc * nc;
+    h->rc_work = h->rc_diag + nc;
+    h->rc_Ainv = q; q += vb;
+    CK(h2d(h, q, host.data(), host.size()));
+    pl.row0 = (const int*)(q + i_row0); pl.halo_ptr = (const int*)(q + i_hp); pl.halo = (const int*)(q + i_halo);
+    pl.agg_rows = (const int*)(q + i_ar); pl.lcol = (const uint16_t*)(q + i_lcol);
+    pl.border = (const uint8_t*)(q + i_bd); pl.off = (const float4*)(q + i_off);
+    h->rc_row0 = (const int*)(q + i_agg0);
+    h->rc_npairs = (int)ab.size();
+    h->rc_ab = (const int2*)(q + i_ab);
+    h->rc_ld = pl.ld;
+    h->rcargs.N = N; h->rcargs.nagg = nagg; h->rcargs.nc = pl.nc;
+    h->rcargs.fixed = h->node_mask; h->rcargs.off = pl.off;
+    h->str = pl;
+    h->str_state = 1;
     return SORS_OK;
 }
 
@@ -1190,10 +1415,10 @@ template <typename VT>
 int build_resident_coarse(SorsHandle* h) {
     const int nc = h->rcargs.nc;
     CK(cudaMemsetAsync(h->rc_Ac, 0, sizeof(double) * ((size_t)nc * nc + nc), h->stream));
-    launch_range_galerkin<VT>(h->rc_npairs, h->rc_ab, h->res.row0, h->row_ptr, h->col, (const VT*)h->H, h->rcargs,
+    launch_range_galerkin<VT>(h->rc_npairs, h->rc_ab, h->rc_row0, h->row_ptr, h->col, (const VT*)h->H, h->rcargs,
                               h->rc_Ac, h->rc_diag, h->stream);
     launch_coarse_invert(nc, h->rc_Ac, h->rc_diag, h->rc_work, h->stream);
-    launch_to_vt_perm<VT>(nc, h->rc_Ac, (VT*)h->rc_Ainv, h->stream);
+    launch_to_vt_perm<VT>(nc, h->rc_ld, h->rc_Ac, (VT*)h->rc_Ainv, h->stream);
     h->rc_ready = true;
     h->tl_refreshes++;
     return SORS_OK;
@@ -1201,32 +1426,46 @@ int build_resident_coarse(SorsHandle* h) {
 
 // The solve as one launch; *ran = false when it cannot be launched here.
 template <typename VT>
-int pcg_resident(SorsHandle* h, double eta, double abs_tol, const double* g, bool* ran) {
-    ResidentArgs<VT> a;
-    a.row_ptr = h->row_ptr; a.diag_slot = h->diag_slot; a.H = (const VT*)h->H; a.g = g ? g : h->g;
-    a.x = (VT*)h->x; a.p0 = (VT*)h->p0; a.p1 = (VT*)h->p1; a.zg = h->res_zg; a.box = h->res_box;
-    a.eta2 = eta * eta; a.abs_tol2 = abs_tol * abs_tol; a.maxit = h->s.pcg_max_iter;
-    a.pflag = h->proj_flag; a.pn = h->proj_n; a.epoch = h->res_epoch; a.sc = h->sc;
-    a.fixed = h->node_mask;
+int pcg_one_launch(SorsHandle* h, double eta, double abs_tol, const double* g, bool* ran) {
+    *ran = false;
+    int st = ensure_resident(h);
+    if (st) return st;
+    if (h->res_state != 1 && (st = ensure_stream(h))) return st;
+    if (h->res_state != 1 && h->str_state != 1) return SORS_OK;
+    const bool coarse = h->res_state == 1 ? h->res.coarse != 0 : true;
     bool refreshed = false;
-    if (h->res.coarse) {
-        if (!h->rc_ready) {
-            int st = build_resident_coarse<VT>(h);
-            if (st) return st;
-            refreshed = true;
-        }
-        a.Ainv = (const VT*)h->rc_Ainv;
+    if (coarse && !h->rc_ready) {
+        if ((st = build_resident_coarse<VT>(h))) return st;
+        refreshed = true;
     }
-    *ran = launch_pcg_resident<VT>(h->res, a, h->stream) == 0;
+    auto fill = [&](auto& a) {
+        a.row_ptr = h->row_ptr; a.diag_slot = h->diag_slot; a.H = (const VT*)h->H; a.g = g ? g : h->g;
+        a.x = (VT*)h->x; a.p0 = (VT*)h->p0; a.p1 = (VT*)h->p1; a.zg = h->res_zg; a.box = h->res_box;
+        a.eta2 = eta * eta; a.abs_tol2 = abs_tol * abs_tol; a.maxit = h->s.pcg_max_iter;
+        a.pflag = h->proj_flag; a.pn = h->proj_n; a.epoch = h->res_epoch; a.sc = h->sc;
+        a.fixed = h->node_mask;
+        a.Ainv = coarse ? (const VT*)h->rc_Ainv : nullptr;
+    };
+    if (h->res_state == 1) {
+        ResidentArgs<VT> a;
+        fill(a);
+        *ran = launch_pcg_resident<VT>(h->res, a, h->stream) == 0;
+        if (!*ran) h->res_state = -1;
+    } else {
+        StreamArgs<VT> a;
+        fill(a);
+        a.ws = (VT*)h->str_ws; a.woff = h->str_woff; a.board = h->str_board;
+        *ran = launch_pcg_stream<VT>(h->str, a, h->stream) == 0;
+        if (!*ran) h->str_state = -1;
+    }
     if (!*ran) {
         cudaGetLastError();
-        h->res_state = -1;
         return SORS_OK;
     }
     CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     if (h->sc_host->status & kFlagTimeout) return fail(SORS_ERR_CUDA, "the PCG blocks did not meet within the limit");
-    if (h->res.coarse) coarse_rate_check(h, refreshed, &h->rc_ref_rate, &h->rc_ready);
+    if (coarse) coarse_rate_check(h, refreshed, &h->rc_ref_rate, &h->rc_ready);
     return SORS_OK;
 }
 
@@ -1236,9 +1475,8 @@ int pcg_solve(SorsHandle* h, double eta, double abs_tol, int* iters, const doubl
     bool ran = false;
     if (h->batch.nmem <= 1) {
         h->tl_active = false;
-        int st = ensure_resident(h);
+        int st = pcg_one_launch<VT>(h, eta, abs_tol, g, &ran);
         if (st) return st;
-        if (h->res_state == 1 && (st = pcg_resident<VT>(h, eta, abs_tol, g, &ran))) return st;
     }
     if (ran) {
         *iters = h->sc_host->it;
@@ -1826,6 +2064,12 @@ int setup_two_level(SorsHandle* h, const double* X) {
         int c[3];
         ab.cell(X + 3 * (size_t)i, c);
         bin[i] = c[0] + dim[0] * (c[1] + dim[1] * c[2]);
+    }
+    // numbering by parts: the parts are the aggregates
+    if (!h->part0.empty()) {
+        remap.assign(h->part0.size(), -1);
+        for (size_t k = 0; k + 1 < h->part0.size(); k++)
+            for (int i = h->part0[k]; i < h->part0[k + 1]; i++) bin[i] = (int)k;
     }
     // aggregates numbered in the order of their lowest node
     int nagg = 0;
@@ -2479,7 +2723,9 @@ int set_device(SorsHandle* h) {
 // within a box the Morton order of the undeformed positions (21 bits per axis,
 // one scale for all axes), so that every aggregate is a contiguous node range.
 // SORS_NO_RENUMBER=1 keeps the caller's numbering (for comparison).
-void locality_order(int N, int E, int nv, const double* X, const int32_t* conn, std::vector<int>& n2o) {
+void number_by_parts(SorsHandle* h, const double* X, std::vector<int>& n2o);
+void locality_order(SorsHandle* h, int N, int E, int nv, const double* X, const int32_t* conn,
+                    std::vector<int>& n2o) {
     std::vector<int> parent(N);
     for (int i = 0; i < N; i++) parent[i] = i;
     auto find = [&](int a) {
@@ -2492,7 +2738,12 @@ void locality_order(int N, int E, int nv, const double* X, const int32_t* conn, 
             if (a != b) parent[std::max(a, b)] = std::min(a, b);
         }
     std::vector<int> root(N);
-    for (int i = 0; i < N; i++) root[i] = find(i);  // the component's lowest index
+    bool one = true;
+    for (int i = 0; i < N; i++) {
+        root[i] = find(i);  // the component's lowest index
+        one = one && root[i] == 0;
+    }
+    if (one && h->parts_form) return number_by_parts(h, X, n2o);
     double lo[3] = {X[0], X[1], X[2]}, hi[3] = {X[0], X[1], X[2]};
     for (int i = 0; i < N; i++)
         for (int k = 0; k < 3; k++) {
@@ -2525,6 +2776,91 @@ void locality_order(int N, int E, int nv, const double* X, const int32_t* conn, 
     std::sort(key.begin(), key.end());
     n2o.resize(N);
     for (int i = 0; i < N; i++) n2o[i] = std::get<3>(key[i]);
+}
+
+// Numbering for the one-launch PCGs: recursive coordinate bisection of the nodes
+// into G ranges of equal size, and of each into A aggregates, each part in Morton
+// order.  Against equal ranges of the box order (parts of several boxes), the same
+// number of coarse unknowns takes 20-30 % fewer iterations: 21k tets 195 -> 151 (64
+// parts), 123k tets 249 -> 188 (148), a hex arm 362 -> 279 (148).
+void number_by_parts(SorsHandle* h, const double* X, std::vector<int>& n2o) {
+    const int N = h->N, G = h->parts_G, A = h->parts_A;
+    n2o.resize(N);
+    for (int i = 0; i < N; i++) n2o[i] = i;
+    h->part0.assign((size_t)G * A + 1, N);
+    double lo[3], hi[3];
+    auto extent = [&](const int* a, const int* b, double* l, double* u) {
+        for (int k = 0; k < 3; k++) { l[k] = 1e300; u[k] = -1e300; }
+        for (; a < b; a++)
+            for (int k = 0; k < 3; k++) {
+                const double x = X[3 * (size_t)*a + k];
+                l[k] = std::min(l[k], x);
+                u[k] = std::max(u[k], x);
+            }
+    };
+    extent(n2o.data(), n2o.data() + N, lo, hi);
+    const double ext = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
+    auto spread = [](uint64_t v) {
+        v &= 0x1fffff;
+        v = (v | v << 32) & 0x1f00000000ffffULL;
+        v = (v | v << 16) & 0x1f0000ff0000ffULL;
+        v = (v | v << 8) & 0x100f00f00f00f00fULL;
+        v = (v | v << 4) & 0x10c30c30c30c30c3ULL;
+        v = (v | v << 2) & 0x1249249249249249ULL;
+        return v;
+    };
+    std::vector<uint64_t> code(N);
+    parallel_for(N, [&](int a, int b) {
+        for (int i = a; i < b; i++) {
+            code[i] = 0;
+            for (int k = 0; k < 3; k++) {
+                const double u = ext > 0 ? (X[3 * (size_t)i + k] - lo[k]) / ext : 0.0;
+                code[i] |= spread((uint64_t)std::min(2097151.0, std::max(0.0, u * 2097151.0))) << k;
+            }
+        }
+    });
+    // nodes [a, b) of n2o into `parts` parts; the first half's size from `head`
+    auto split = [&](int a, int b, int m) {
+        double l[3], u[3];
+        extent(n2o.data() + a, n2o.data() + b, l, u);
+        int ax = 0;
+        for (int k = 1; k < 3; k++)
+            if (u[k] - l[k] > u[ax] - l[ax]) ax = k;
+        std::nth_element(n2o.begin() + a, n2o.begin() + m, n2o.begin() + b, [&](int p, int q) {
+            const double x = X[3 * (size_t)p + ax], y = X[3 * (size_t)q + ax];
+            return x < y || (x == y && p < q);
+        });
+    };
+    // aggregates of a range: whole warps of rows each
+    std::function<void(int, int, int, int, int)> leaves = [&](int a, int b, int k0, int k1, int L) {
+        if (k1 - k0 == 1) {
+            h->part0[k0] = a;
+            std::sort(n2o.begin() + a, n2o.begin() + b,
+                      [&](int p, int q) { return code[p] < code[q] || (code[p] == code[q] && p < q); });
+            return;
+        }
+        const int half = (k1 - k0) / 2, m = std::min(b, a + half * L);
+        if (m > a && m < b) split(a, b, m);
+        leaves(a, m, k0, k0 + half, L);
+        leaves(m, b, k0 + half, k1, L);
+    };
+    std::function<void(int, int, int, int, int)> ranges = [&](int a, int b, int g0, int g1, int depth) {
+        if (g1 - g0 == 1) {
+            leaves(a, b, g0 * A, g0 * A + A, part_rows(b - a, A));
+            return;
+        }
+        const int half = (g1 - g0) / 2, m = a + (int)((int64_t)(b - a) * half / (g1 - g0));
+        if (m > a && m < b) split(a, b, m);
+        if (depth < 3 && b - a > 20000) {
+            std::thread t([&]() { ranges(a, m, g0, g0 + half, depth + 1); });
+            ranges(m, b, g0 + half, g1, depth + 1);
+            t.join();
+        } else {
+            ranges(a, m, g0, g0 + half, depth);
+            ranges(m, b, g0 + half, g1, depth);
+        }
+    };
+    ranges(0, N, 0, G, 0);
 }
 
 // Caller-numbered DOF vector (host or device) -> internal device vector.
@@ -2628,6 +2964,11 @@ int sors_create(const double* X, int32_t n_nodes, const int32_t* conn, int32_t n
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(fail(SORS_ERR_CUDA, "stream creation failed"));
     const int N = n_nodes, E = n_elems, nv = nodes_per_elem;
+    // two_level 2 ("auto"), for the launch-per-kernel PCG: on for meshes of 20,000 nodes
+    // or more, where the coarse correction's extra kernels pay for themselves
+    h->tl_req = h->s.two_level;
+    if (h->s.two_level == 2) h->s.two_level = N >= 20000 ? 1 : 0;
+    choose_parts(h);
     // the handle's node numbering (locality order); the rest of the set-up
     // reads the renumbered positions and connectivity
     std::vector<double> X_int, rho_int, youngs_int, poisson_int;
@@ -2635,7 +2976,7 @@ int sors_create(const double* X, int32_t n_nodes, const int32_t* conn, int32_t n
     {
         const char* env = getenv("SORS_NO_RENUMBER");
         const bool off = env && *env && *env != '0';
-        if (!off) locality_order(N, E, nv, X, conn, h->n2o);
+        if (!off) locality_order(h, N, E, nv, X, conn, h->n2o);
         h->renum = false;
         if (!off)
             for (int i = 0; i < N && !h->renum; i++) h->renum = h->n2o[i] != i;
@@ -2726,16 +3067,10 @@ int sors_create(const double* X, int32_t n_nodes, const int32_t* conn, int32_t n
     CK(h2d(h, h->q, X, nd * sizeof(double)));
     h->mask_h.assign(N, 0);
     if ((st = upload(h, &h->node_mask, h->mask_h.data(), (size_t)N))) return bail(st);
-    // two_level 2 ("auto"): on for meshes of 20,000 nodes or more, where the
-    // coarse correction's three extra kernels per iteration pay for themselves
-    h->tl_req = h->s.two_level;
-    if (h->s.two_level == 2) h->s.two_level = N >= 20000 ? 1 : 0;
     size_t hs = hsize(h);
-    // meshes the one-launch PCG may take (about 300 KB of matrix per SM) set it up at
-    // a solve that needs it
-    if (h->s.two_level && (size_t)h->nnzb * 9 * hs > ((size_t)kResidentMaxBlocks * 300 << 10) &&
-        (st = setup_two_level(h, X)))
-        return bail(st);
+    // meshes that a one-launch PCG takes set the two-level preconditioner of the others
+    // up at a solve that needs it
+    if (h->s.two_level && !h->parts_form && (st = setup_two_level(h, X))) return bail(st);
     // 160 bytes of padding: the SpMV reads values in 144-byte groups, the last of
     // which may run past the last block
     if ((st = dalloc(h, &h->H, (size_t)h->nnzb * 9 * hs + 160))) return bail(st);

@@ -3117,20 +3117,20 @@ void launch_to_vt_pad(int nc, int ld, const double* in, VT* out, cudaStream_t st
 }
 
 template <typename VT>
-__global__ void k_to_vt_perm(int nc, const double* __restrict__ in, VT* __restrict__ out) {
+__global__ void k_to_vt_perm(int nc, int ld, const double* __restrict__ in, VT* __restrict__ out) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)nc * nc) return;
-    const int r = (int)(t / nc), k = (int)(t - (long long)r * nc), G = nc / 6, m = k / G, b = k - m * G;
-    out[t] = (VT)in[(size_t)r * nc + 6 * b + m];
+    if (t >= (long long)nc * ld) return;
+    const int r = (int)(t / ld), k = (int)(t - (long long)r * ld), n = nc / 6, m = k / n, b = k - m * n;
+    out[t] = k < nc ? (VT)in[(size_t)r * nc + 6 * b + m] : VT(0);
 }
 template <typename VT>
-void launch_to_vt_perm(int nc, const double* in, VT* out, cudaStream_t st) {
+void launch_to_vt_perm(int nc, int ld, const double* in, VT* out, cudaStream_t st) {
     if (nc == 0) return;
-    k_to_vt_perm<VT><<<(int)(((long long)nc * nc + 255) / 256), 256, 0, st>>>(nc, in, out);
+    k_to_vt_perm<VT><<<(int)(((long long)nc * ld + 255) / 256), 256, 0, st>>>(nc, ld, in, out);
     counted();
 }
-template void launch_to_vt_perm<float>(int, const double*, float*, cudaStream_t);
-template void launch_to_vt_perm<double>(int, const double*, double*, cudaStream_t);
+template void launch_to_vt_perm<float>(int, int, const double*, float*, cudaStream_t);
+template void launch_to_vt_perm<double>(int, int, const double*, double*, cudaStream_t);
 template void launch_to_vt_pad<float>(int, int, const double*, float*, cudaStream_t);
 template void launch_to_vt_pad<double>(int, int, const double*, double*, cudaStream_t);
 template void launch_tl_update_restrict<float>(const CoarseArgs&, const float*, const float*, float*, float*,

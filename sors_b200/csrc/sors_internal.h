@@ -215,6 +215,51 @@ struct ResidentArgs {
     unsigned* epoch = nullptr;          // grid form: the last epoch used
     DevScalars* sc = nullptr;
 };
+// A whole two-level PCG solve in one launch with the matrix streaming through
+// shared memory (pcg_stream.cu): G blocks, block b owning the rows [row0[b],
+// row0[b + 1]), A aggregates of agg_rows[b] consecutive rows each.
+constexpr int kStreamMaxAgg = 4;
+struct StreamPlan {
+    int G = 0, A = 1, N = 0;
+    int lpr = 4;                        // lanes per row
+    int nc = 0, ld = 0;                 // coarse unknowns 6 A G, leading dimension of their inverse
+    int max_rows = 0, max_cols = 0, max_halo = 0;
+    int group_bytes = 0, depth = 2;     // ring slot: four rows' matrix blocks, column indices, offsets; slots per warp
+    int slot_col = 0, slot_off = 0;     // byte offsets in a slot
+    int a_shared = 0;                   // the block's rows of the coarse inverse are kept in shared memory
+    int evict_first = 0;                // the matrix does not fit in L2
+    const int* row0 = nullptr;
+    const int* halo_ptr = nullptr;
+    const int* halo = nullptr;          // border columns (nodes)
+    const int* agg_rows = nullptr;      // per block, a multiple of 32
+    const uint16_t* lcol = nullptr;
+    const uint8_t* border = nullptr;    // per node: some other range reads its z
+    const float4* off = nullptr;
+};
+template <typename VT>
+struct StreamArgs {
+    const int* row_ptr = nullptr;
+    const int* diag_slot = nullptr;
+    const VT* H = nullptr;
+    const double* g = nullptr;
+    VT *x = nullptr, *p0 = nullptr, *p1 = nullptr;
+    VT* ws = nullptr;                   // 18 N: x, r, z, q (3 N each), inverse diagonal blocks (6 N), by component
+    float4* woff = nullptr;             // N: off with the nodes' flags
+    const VT* Ainv = nullptr;           // row 6 a + m, column m nagg + a for unknown m of aggregate a
+    double eta2 = 0.0, abs_tol2 = 0.0;
+    int maxit = 0;
+    const uint8_t* fixed = nullptr;
+    const uint8_t* pflag = nullptr;
+    const double4* pn = nullptr;
+    unsigned long long *zg = nullptr, *box = nullptr;
+    unsigned long long* board = nullptr;  // three boards of nc entries, two words each
+    unsigned* epoch = nullptr;
+    DevScalars* sc = nullptr;
+};
+size_t stream_smem(const StreamPlan& pl, int vsize);
+template <typename VT>
+int launch_pcg_stream(const StreamPlan& pl, const StreamArgs<VT>& a, cudaStream_t st);
+
 size_t resident_smem(const ResidentPlan& pl, int vsize, int res);
 // Returns 0 or the CUDA error of the launch.
 template <typename VT>
@@ -251,9 +296,9 @@ constexpr int kCoarsePanel = 32;
 inline size_t coarse_work(int nc) { return (size_t)2 * kCoarsePanel * nc + kCoarsePanel * kCoarsePanel; }
 template <typename VT>
 void launch_to_vt_pad(int nc, int ld, const double* in, VT* out, cudaStream_t st);
-// column 6 b + m of `in` as column m nagg + b of `out` (the one-launch PCG's order)
+// column 6 b + m of `in` as column m nagg + b of `out` (the one-launch PCGs' order)
 template <typename VT>
-void launch_to_vt_perm(int nc, const double* in, VT* out, cudaStream_t st);
+void launch_to_vt_perm(int nc, int ld, const double* in, VT* out, cudaStream_t st);
 template <typename VT>
 void launch_coarse_restrict(const CoarseArgs& c, const VT* r, double* yc, cudaStream_t st);
 template <typename VT>
