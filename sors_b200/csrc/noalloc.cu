@@ -38,10 +38,10 @@
 namespace {
 
 constexpr int kNoAllocThreads = 256;
-constexpr int kNoAllocPerThread = 4;
-constexpr int kNoAllocElemsPerBlock = kNoAllocThreads * kNoAllocPerThread;  // 1024
+constexpr int kNoAllocPerThread = 4;  // elements of a thread at most
 constexpr int kNoAllocMaxBlocks = 8192;
-constexpr long long kNoAllocMaxElems = (long long)kNoAllocMaxBlocks * kNoAllocElemsPerBlock;  // 8,388,608
+constexpr long long kNoAllocMaxElems =
+    (long long)kNoAllocMaxBlocks * kNoAllocThreads * kNoAllocPerThread;  // 8,388,608
 
 // [0, kNoAllocMaxBlocks): block partial sums; [kNoAllocMaxBlocks]: completion counter
 // (stored in the first 4 bytes of the slot), padded to 256 bytes.
@@ -57,8 +57,11 @@ int noalloc_fail(int code, const std::string& msg) {
     return code;
 }
 
+// per_thread elements per thread: one while the scratch has a partial sum for
+// every 256 elements (61,440 tets on 60 blocks of four elements a thread left more
+// than half of the SMs without work and each thread four element latencies long).
 template <int NV>
-__global__ void __launch_bounds__(kNoAllocThreads) k_elem_energy_noalloc(int E, const double* __restrict__ Xg,
+__global__ void __launch_bounds__(kNoAllocThreads) k_elem_energy_noalloc(int E, int per_thread, const double* __restrict__ Xg,
                                                                          const double* __restrict__ qg,
                                                                          const int* __restrict__ conn,
                                                                          const double* __restrict__ youngs,
@@ -69,8 +72,8 @@ __global__ void __launch_bounds__(kNoAllocThreads) k_elem_energy_noalloc(int E, 
     __shared__ double sh[kNoAllocThreads / 32];
     __shared__ bool am_last;
     double acc = 0.0;
-    const int e0 = blockIdx.x * kNoAllocElemsPerBlock;
-    for (int k = 0; k < kNoAllocPerThread; k++) {
+    const int e0 = blockIdx.x * kNoAllocThreads * per_thread;
+    for (int k = 0; k < per_thread; k++) {
         const int e = e0 + k * kNoAllocThreads + threadIdx.x;
         if (e >= E) break;
         double X[NV][3], x[NV][3];
@@ -204,12 +207,13 @@ int sors_elem_energy_noalloc(const double* X_device, const double* q_device, con
     // the completion counter must start at zero
     e = cudaMemsetAsync(scratch + (size_t)kNoAllocMaxBlocks * sizeof(double), 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return noalloc_fail(SORS_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-    const int blocks = (n_elems + kNoAllocElemsPerBlock - 1) / kNoAllocElemsPerBlock;
+    const int per_thread = n_elems <= kNoAllocMaxBlocks * kNoAllocThreads ? 1 : kNoAllocPerThread;
+    const int blocks = (n_elems + kNoAllocThreads * per_thread - 1) / (kNoAllocThreads * per_thread);
     if (nodes_per_elem == 4)
-        k_elem_energy_noalloc<4><<<blocks, kNoAllocThreads, 0, s>>>(n_elems, X_device, q_device, conn_device,
+        k_elem_energy_noalloc<4><<<blocks, kNoAllocThreads, 0, s>>>(n_elems, per_thread, X_device, q_device, conn_device,
                                                                     youngs_device, poisson_device, scratch, out_device);
     else
-        k_elem_energy_noalloc<8><<<blocks, kNoAllocThreads, 0, s>>>(n_elems, X_device, q_device, conn_device,
+        k_elem_energy_noalloc<8><<<blocks, kNoAllocThreads, 0, s>>>(n_elems, per_thread, X_device, q_device, conn_device,
                                                                     youngs_device, poisson_device, scratch, out_device);
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(SORS_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
