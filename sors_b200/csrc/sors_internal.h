@@ -425,6 +425,8 @@ void launch_gather_dofs(int N, const double* src, const int* idx, double* dst, c
 void launch_cfl(int E, int nv, const double* q, const int* conn, int n, const double* vPrev, double* partials,
                 DevScalars* sc, cudaStream_t st);
 template <typename HT>
+void launch_blocks_out(long long b0, long long n, const int* blk, const HT* H, double* out, cudaStream_t st);
+template <typename HT>
 void launch_spmv_plain(int N, const int* row_ptr, const int* col, const HT* H, long long nnzb, const double* x,
                        double* y, cudaStream_t st);
 

@@ -139,3 +139,20 @@ def test_capped_handle_and_concurrent_streams():
         t.join()
     for k, _ in jobs:
         assert np.array_equal(out[("alone", k)], out[("mix", k)])
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("mixed", 1e-5)])
+def test_hessian_blocks_in_two_pieces(oracle, precision, tol):
+    """compute_hessian of a mesh with more blocks than one copy takes (about 250,000,
+    against 233,016), in the caller's order, against the oracle.  FP64 to the assembly's
+    1e-10; FP32 blocks to 1e-5 of the largest entry (60 items at 6e-8 each, doubled)."""
+    from tests.helpers import make_pair
+    X = meshes.grid_nodes(25, 25, 25, (0.1, 0.1, 0.1))
+    T = meshes.kuhn_tet_elements(25, 25, 25)
+    rng = np.random.default_rng(3)
+    q = (X @ (np.eye(3) + rng.uniform(-0.05, 0.05, (3, 3))).T).ravel()
+    en, _, o, _ = make_pair(X, T, project=False, precision=precision)
+    H = en.compute_hessian(q, 1e-3)
+    Ho, _ = o.hessian_csr(q, 1e-3)
+    d = H - Ho
+    assert np.abs(d.data).max() <= tol * np.abs(Ho.data).max()
