@@ -1422,23 +1422,26 @@ int build_resident_coarse(SorsHandle* h) {
     launch_coarse_invert(nc, h->rc_Ac, h->rc_diag, h->rc_work, h->stream);
     launch_to_vt_perm<VT>(nc, h->rc_ld, h->rc_Ac, (VT*)h->rc_Ainv, h->stream);
     h->rc_ready = true;
+    h->rc_ref_rate = -1.0;
     h->tl_refreshes++;
     return SORS_OK;
 }
 
-// The solve as one launch; *ran = false when it cannot be launched here.
+// The solve as one launch, left running; *ran = false when it cannot be launched
+// here, *refreshed: the coarse operator was rebuilt.  nf: the forcing term from
+// the device (null: eta and abs_tol).
 template <typename VT>
-int pcg_one_launch(SorsHandle* h, double eta, double abs_tol, const double* g, bool* ran) {
-    *ran = false;
+int pcg_one_launch(SorsHandle* h, double eta, double abs_tol, const double* g, const NewtonForcing* nf, bool* ran,
+                   bool* refreshed) {
+    *ran = *refreshed = false;
     int st = ensure_resident(h);
     if (st) return st;
     if (h->res_state != 1 && (st = ensure_stream(h))) return st;
     if (h->res_state != 1 && h->str_state != 1) return SORS_OK;
     const bool coarse = h->res_state == 1 ? h->res.coarse != 0 : true;
-    bool refreshed = false;
     if (coarse && !h->rc_ready) {
         if ((st = build_resident_coarse<VT>(h))) return st;
-        refreshed = true;
+        *refreshed = true;
     }
     auto fill = [&](auto& a) {
         a.row_ptr = h->row_ptr; a.diag_slot = h->diag_slot; a.H = (const VT*)h->H; a.g = g ? g : h->g;
@@ -1447,6 +1450,7 @@ int pcg_one_launch(SorsHandle* h, double eta, double abs_tol, const double* g, b
         a.pflag = h->proj_flag; a.pn = h->proj_n; a.epoch = h->res_epoch; a.sc = h->sc;
         a.fixed = h->node_mask;
         a.Ainv = coarse ? (const VT*)h->rc_Ainv : nullptr;
+        if (nf) a.nf = *nf;
     };
     if (h->res_state == 1) {
         ResidentArgs<VT> a;
@@ -1460,35 +1464,38 @@ int pcg_one_launch(SorsHandle* h, double eta, double abs_tol, const double* g, b
         *ran = launch_pcg_stream<VT>(h->str, a, h->stream) == 0;
         if (!*ran) h->str_state = -1;
     }
-    if (!*ran) {
-        cudaGetLastError();
-        return SORS_OK;
-    }
-    CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    if (!*ran) cudaGetLastError();
+    return SORS_OK;
+}
+
+// After a one-launch solve, its scalars in sc_host.
+template <typename VT>
+int pcg_one_launch_done(SorsHandle* h, bool refreshed, int* iters) {
     if (h->sc_host->status & kFlagTimeout) return fail(SORS_ERR_CUDA, "the PCG blocks did not meet within the limit");
-    if (coarse) coarse_rate_check(h, refreshed, &h->rc_ref_rate, &h->rc_ready);
+    if (h->res_state == 1 ? h->res.coarse != 0 : true)
+        coarse_rate_check(h, refreshed, &h->rc_ref_rate, &h->rc_ready);
+    *iters = h->sc_host->it;
+    if (!h->sc_host->breakdown) return SORS_OK;
+    int st = record_curvature<VT>(h);
+    if (st) return st;
+    if (h->sc_host->it == 0 && !(h->s.project_spd == 2 && !h->proj_fallback))
+        return fail(SORS_ERR_PCG_BREAKDOWN, "PCG breakdown: the Hessian is not positive definite");
     return SORS_OK;
 }
 
 template <typename HT, typename VT>
 int pcg_solve(SorsHandle* h, double eta, double abs_tol, int* iters, const double* g = nullptr) {
     static_assert(std::is_same<HT, VT>::value, "PCG vectors have the matrix's type");
-    bool ran = false;
     if (h->batch.nmem <= 1) {
         h->tl_active = false;
-        int st = pcg_one_launch<VT>(h, eta, abs_tol, g, &ran);
+        bool ran, refreshed;
+        int st = pcg_one_launch<VT>(h, eta, abs_tol, g, nullptr, &ran, &refreshed);
         if (st) return st;
-    }
-    if (ran) {
-        *iters = h->sc_host->it;
-        if (h->sc_host->breakdown) {
-            int st = record_curvature<VT>(h);
-            if (st) return st;
-            if (h->sc_host->it == 0 && !(h->s.project_spd == 2 && !h->proj_fallback))
-                return fail(SORS_ERR_PCG_BREAKDOWN, "PCG breakdown: the Hessian is not positive definite");
+        if (ran) {
+            CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
+            CK(cudaStreamSynchronize(h->stream));
+            return pcg_one_launch_done<VT>(h, refreshed, iters);
         }
-        return SORS_OK;
     }
     launch_block_jacobi<HT, VT>(h->N, h->row_ptr, h->diag_slot, (const HT*)h->H, h->nnzb, (VT*)h->Minv, h->stream);
     if (h->batch.nmem > 1) return pcg_solve_members<HT, VT>(h, eta, abs_tol, iters, g);
@@ -1843,6 +1850,23 @@ int minimize(SorsHandle* h, double dt, SorsStepStats* stats) {
                            prev_eta * prev_g <= 1e3 * res_tol;
         if ((st = eval_system<HT>(h, dt, want_hess && !probe))) return st;
         if (want_hess && !probe) have_hess = true;
+        // Full Newton steps solved by one launch: the solve (its forcing term formed on
+        // the device) and the update follow the evaluation without a round trip to the
+        // host, which reads all scalars once; both are skipped on the device where the
+        // decisions below end the iteration before them.
+        NewtonForcing nf;
+        nf.on = 1; nf.prev_g = prev_g; nf.prev_eta = prev_eta; nf.res_tol = res_tol;
+        nf.floor = mixed(h) ? std::max(h->s.pcg_rel_tol, 1e-6) : h->s.pcg_rel_tol;
+        bool ahead = m == 0 && !probe && h->batch.nmem <= 1 && h->s.linear_solver == 0 &&
+                     !(h->s.project_spd == 2 && h->s.newton_safeguard);
+        bool refreshed = false;
+        if (ahead) {
+            h->tl_active = false;
+            if ((st = pcg_one_launch<VT>(h, 0.0, 0.0, nullptr, &nf, &ahead, &refreshed))) return st;
+            if (ahead)
+                launch_newton_update<VT>(n, (const VT*)h->x, 1.0, h->q, h->q, h->partials, h->sc, 6, h->stream,
+                                         h->s.project_spd == 2 && !h->proj_fallback ? 2 : 1);
+        }
         CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
         if (h->sc_host->status & kFlagInverted)
@@ -1859,27 +1883,24 @@ int minimize(SorsHandle* h, double dt, SorsStepStats* stats) {
         // forcing term: Eisenstat-Walker choice 2 with its safeguard, never
         // solving below what the residual target needs, floored at pcg_rel_tol
         // (and at 1e-6 for FP32 PCG vectors)
-        double eta = 0.5;
-        if (prev_g > 0.0) {
-            const double ratio = gn / prev_g;
-            eta = 0.9 * ratio * ratio;
-            const double safe = 0.9 * prev_eta * prev_eta;
-            if (safe > 0.1) eta = std::max(eta, safe);
-            eta = std::min(eta, 0.5);
-        }
-        if (res_tol > 0.0) eta = std::max(eta, std::min(0.5, 0.5 * res_tol / gn));
-        eta = std::max(eta, mixed(h) ? std::max(h->s.pcg_rel_tol, 1e-6) : h->s.pcg_rel_tol);
+        const double eta = newton_forcing(nf, gn);
         prev_g = gn;
         prev_eta = eta;
         int pit = 0;
-        if ((st = newton_solve<HT, VT>(h, dt, eta, res_tol > 0.0 ? 0.1 * res_tol : 0.0, &pit))) return st;
+        if (ahead) {
+            if ((st = pcg_one_launch_done<VT>(h, refreshed, &pit))) return st;
+        } else if ((st = newton_solve<HT, VT>(h, dt, eta, res_tol > 0.0 ? 0.1 * res_tol : 0.0, &pit))) {
+            return st;
+        }
         if (stats) stats->pcg_iters += pit;
+        bool updated = ahead;
         if (h->s.project_spd == 2 && !h->proj_fallback && h->sc_host->breakdown) {
             // negative curvature in the exact Hessian: solve this iteration with the projected one
             h->proj_fallback = true;
             if ((st = eval_system<HT>(h, dt, true))) return st;
             if ((st = pcg_solve<HT, VT>(h, eta, res_tol > 0.0 ? 0.1 * res_tol : 0.0, &pit))) return st;
             if (stats) stats->pcg_iters += pit;
+            updated = false;
         }
         double alpha = 1.0;
         if (m == 1) {
@@ -1898,7 +1919,7 @@ int minimize(SorsHandle* h, double dt, SorsStepStats* stats) {
                 alpha *= 0.5;
             }
             if (!accepted) return fail(SORS_ERR_LINESEARCH, "line search did not find a decrease");
-        } else {
+        } else if (!updated) {
             CK(cudaMemcpyAsync(h->q0, h->q, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream));
             launch_newton_update<VT>(n, (const VT*)h->x, 1.0, h->q, h->q0, h->partials, h->sc, 6, h->stream);
             if (m == 0 && h->s.project_spd == 2 && h->s.newton_safeguard) {
@@ -1919,8 +1940,10 @@ int minimize(SorsHandle* h, double dt, SorsStepStats* stats) {
                 }
             }
         }
-        CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        if (!updated) {
+            CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
+            CK(cudaStreamSynchronize(h->stream));
+        }
         double dxn = sqrt(h->sc_host->dxnorm2) / alpha;
         if (stats) stats->dx_norm = dxn;
         if (verbose())

@@ -2302,7 +2302,9 @@ void launch_pcg_update(int N, const VT* p, const VT* qv, const VT* Minv, VT* x, 
 template <typename VT>
 __global__ void __launch_bounds__(kRedThreads) k_newton_update(int n, const VT* dx, double alpha, double* q,
                                                                 const double* q0, double* partials, DevScalars* sc,
-                                                                int counter) {
+                                                                int counter, int gate) {
+    // gate 1: not after a skipped solve; 2: nor after one that met negative curvature
+    if (gate && (sc->skip || (gate == 2 && sc->breakdown))) return;
     double acc[1] = {0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double d = alpha * (double)dx[i];
@@ -2315,8 +2317,8 @@ __global__ void __launch_bounds__(kRedThreads) k_newton_update(int n, const VT* 
 
 template <typename VT>
 void launch_newton_update(int n, const VT* dx, double alpha, double* q, const double* q0, double* partials,
-                          DevScalars* sc, int counter, cudaStream_t st) {
-    k_newton_update<VT><<<red_grid(n, 4), kRedThreads, 0, st>>>(n, dx, alpha, q, q0, partials, sc, counter);
+                          DevScalars* sc, int counter, cudaStream_t st, int gate) {
+    k_newton_update<VT><<<red_grid(n, 4), kRedThreads, 0, st>>>(n, dx, alpha, q, q0, partials, sc, counter, gate);
     counted();
 }
 
@@ -3241,9 +3243,9 @@ template void launch_pcg_update<double>(int, const double*, const double*, const
 template void launch_pcg_update<float>(int, const float*, const float*, const float*, float*, float*, float*,
                                        const uint8_t*, const double4*, double*, DevScalars*, cudaStream_t);
 template void launch_newton_update<double>(int, const double*, double, double*, const double*, double*, DevScalars*,
-                                           int, cudaStream_t);
+                                           int, cudaStream_t, int);
 template void launch_newton_update<float>(int, const float*, double, double*, const double*, double*, DevScalars*, int,
-                                          cudaStream_t);
+                                          cudaStream_t, int);
 template void launch_dot_gdx<double>(int, const double*, const double*, double*, DevScalars*, cudaStream_t);
 template void launch_dot_gdx<float>(int, const double*, const float*, double*, DevScalars*, cudaStream_t);
 template void launch_spmv_plain<double>(int, const int*, const int*, const double*, long long, const double*,

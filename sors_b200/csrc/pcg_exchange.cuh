@@ -179,6 +179,29 @@ __device__ __forceinline__ bool exchange(double (&v)[NSUM ? NSUM : 1], Scratch* 
     }
 }
 
+// Tolerances of a solve; false when the Newton iteration ends before it (the
+// whole grid agrees: the scalars read here are not written by this launch).
+template <typename Args>
+__device__ __forceinline__ bool solve_tolerances(const Args& a, double& eta2, double& abs2) {
+    eta2 = a.eta2;
+    abs2 = a.abs_tol2;
+    if (!a.nf.on) return true;
+    const double gn = sqrt(a.sc->gnorm2);
+    if ((a.sc->status & kFlagInverted) || !(gn == gn) || (a.nf.res_tol > 0.0 && gn < a.nf.res_tol)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            a.sc->skip = 1;
+            a.sc->it = 0;
+            a.sc->breakdown = 0;
+            a.sc->done = 1;
+        }
+        return false;
+    }
+    const double eta = newton_forcing(a.nf, gn);
+    eta2 = eta * eta;
+    abs2 = a.nf.res_tol > 0.0 ? 0.01 * a.nf.res_tol * a.nf.res_tol : 0.0;
+    return true;
+}
+
 template <typename VT>
 __device__ __forceinline__ void project(unsigned f, const double4* pn, VT (&y)[3]) {
     if (!f) return;

@@ -96,6 +96,8 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int P = Lay<VT>::P, Z = Lay<VT>::Z;
     constexpr int NG = kT / LPR;  // groups of lanes
+    double eta2, abs_tol2;
+    if (!solve_tolerances(a, eta2, abs_tol2)) return;
     Scratch* sh = reinterpret_cast<Scratch*>(smem);
     const Off o = offsets<VT>(pl);
     VT* sp = reinterpret_cast<VT*>(smem + o.sp);
@@ -326,7 +328,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
     par1 ^= 1u;
     double rz = acc[0], rr = acc[1], pq = 0.0, alpha = 0.0, beta = 0.0;
     const double bnorm2 = rr;
-    const double te = a.eta2 * rr, tol2 = te > a.abs_tol2 ? te : a.abs_tol2;
+    const double te = eta2 * rr, tol2 = te > abs_tol2 ? te : abs_tol2;
     int it = 0, breakdown = 0;
     bool done = !ok || rr <= tol2 || a.maxit <= 0;
     // threads without a row take the border columns first
@@ -493,7 +495,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
         DevScalars* sc = a.sc;
         sc->rz = rz; sc->rr = rr; sc->bnorm2 = bnorm2; sc->tol2 = tol2; sc->pq = pq;
         sc->alpha = breakdown ? 0.0 : alpha; sc->beta = beta;
-        sc->it = it; sc->maxit = a.maxit; sc->breakdown = breakdown; sc->done = 1;
+        sc->it = it; sc->maxit = a.maxit; sc->breakdown = breakdown; sc->done = 1; sc->skip = 0;
         if (sh->abort) sc->status |= kFlagTimeout;
         if (!CL) *a.epoch = epoch;
     }

@@ -84,6 +84,8 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
     constexpr int kGR = 32 / kLPR;  // rows per group
     constexpr int P = Lay<VT>::P, Z = Lay<VT>::Z;
     constexpr int BB = 9 * (int)sizeof(VT);  // bytes of a matrix block
+    double eta2, abs_tol2;
+    if (!solve_tolerances(a, eta2, abs_tol2)) return;
     Scratch* sh = reinterpret_cast<Scratch*>(smem);
     const SOff o = soffsets<VT>(pl);
     double* zc = reinterpret_cast<double*>(smem + o.zc);      // 6 A rows, two partial sums each
@@ -369,7 +371,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
     ok = exchange<1, 2, 2, false>(acc, sh, G, ++epoch, a.box, 0u, 0, nullptr) && ok;
     double rz = acc[0], rr = acc[1], pq = 0.0, alpha = 0.0, beta = 0.0;
     const double bnorm2 = rr;
-    const double te = a.eta2 * rr, tol2 = te > a.abs_tol2 ? te : a.abs_tol2;
+    const double te = eta2 * rr, tol2 = te > abs_tol2 ? te : abs_tol2;
     int it = 0, breakdown = 0, flip = 0;
     bool done = !ok || rr <= tol2 || a.maxit <= 0;
     while (!done) {
@@ -522,7 +524,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
         DevScalars* sc = a.sc;
         sc->rz = rz; sc->rr = rr; sc->bnorm2 = bnorm2; sc->tol2 = tol2; sc->pq = pq;
         sc->alpha = breakdown ? 0.0 : alpha; sc->beta = beta;
-        sc->it = it; sc->maxit = a.maxit; sc->breakdown = breakdown; sc->done = 1;
+        sc->it = it; sc->maxit = a.maxit; sc->breakdown = breakdown; sc->done = 1; sc->skip = 0;
         if (sh->abort) sc->status |= kFlagTimeout;
         *a.epoch = epoch;
     }

@@ -35,6 +35,7 @@ struct DevScalars {
     // PCG
     double rz, pq, alpha, beta, rr, tol2, bnorm2;
     int it, done, maxit, breakdown;
+    int skip;            // the Newton iteration ends before its solve (NewtonForcing)
     // MINRES (Lanczos vectors with Givens QR, minres.cu): gamma_{j-1},
     // gamma_j, delta_j, c_{j-1}, c_j, s_{j-1}, s_j and eta (the preconditioned
     // residual norm, signed); the solution update the last iteration left
@@ -173,6 +174,29 @@ void launch_bpcg_iter(const BatchArgs& b, const int* row_ptr, const int* col, co
                       const VT* z_in, const VT* p_old, VT* p_new, VT* qv, VT* x, VT* r, VT* z,
                       const uint8_t* pflag, const double4* pn, cudaStream_t st);
 
+// Forcing term of a Newton iteration formed on the device from ||g|| in the
+// scalars, so that the host need not read it before the solve is launched: as
+// minimize() forms it.  The solve and the update after it are skipped (skip = 1)
+// when the iteration ends at the gradient: an inverted element, NaN, converged.
+struct NewtonForcing {
+    int on = 0;
+    double prev_g = -1.0, prev_eta = 0.5, res_tol = 0.0, floor = 0.0;
+};
+__host__ __device__ inline double newton_forcing(const NewtonForcing& f, double gn) {
+    double eta = 0.5;
+    if (f.prev_g > 0.0) {
+        const double ratio = gn / f.prev_g, safe = 0.9 * f.prev_eta * f.prev_eta;
+        eta = 0.9 * ratio * ratio;
+        if (safe > 0.1 && safe > eta) eta = safe;
+        if (eta > 0.5) eta = 0.5;
+    }
+    if (f.res_tol > 0.0) {
+        const double need = 0.5 * f.res_tol / gn;
+        if (need > eta) eta = need < 0.5 ? need : (eta > 0.5 ? eta : 0.5);
+    }
+    return eta > f.floor ? eta : f.floor;
+}
+
 // A whole block-Jacobi PCG solve in one launch (pcg_resident.cu): G blocks of
 // kResidentThreads threads, block b owning the rows [row0[b], row0[b + 1]).
 constexpr int kResidentThreads = 512;
@@ -205,6 +229,7 @@ struct ResidentArgs {
     VT* x = nullptr;
     VT *p0 = nullptr, *p1 = nullptr;    // receive the direction of a breakdown (by the parity of the iteration)
     double eta2 = 0.0, abs_tol2 = 0.0;
+    NewtonForcing nf;                   // on: in place of eta2 and abs_tol2
     int maxit = 0;
     const uint8_t* pflag = nullptr;     // constraint projection (null: none)
     const double4* pn = nullptr;
@@ -247,6 +272,7 @@ struct StreamArgs {
     float4* woff = nullptr;             // N: off with the nodes' flags
     const VT* Ainv = nullptr;           // row 6 a + m, column m nagg + a for unknown m of aggregate a
     double eta2 = 0.0, abs_tol2 = 0.0;
+    NewtonForcing nf;                   // on: in place of eta2 and abs_tol2
     int maxit = 0;
     const uint8_t* fixed = nullptr;
     const uint8_t* pflag = nullptr;
@@ -415,7 +441,7 @@ void launch_pair_axpy(int np, const int2* ij, const double4* coef, double* y, cu
 void launch_axpy(int n, double alpha, const double* x, double* y, cudaStream_t st);
 template <typename VT>
 void launch_newton_update(int n, const VT* dx, double alpha, double* q, const double* q0, double* partials,
-                          DevScalars* sc, int counter, cudaStream_t st);
+                          DevScalars* sc, int counter, cudaStream_t st, int gate = 0);
 template <typename VT>
 void launch_dot_gdx(int n, const double* g, const VT* dx, double* partials, DevScalars* sc, cudaStream_t st);
 void launch_update_state(int n, const double* q, double* qPrev, double* vPrev, double* gPrev,
