@@ -286,6 +286,20 @@ cudaError_t h2d(SorsHandle* h, void* dst, const void* src, size_t bytes) {
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream);
     return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
 }
+// From this library's own pageable arrays: the copy is staged when the call
+// returns, so the array may change, and later work on the stream is ordered.
+cudaError_t h2d_staged(SorsHandle* h, void* dst, const void* src, size_t bytes) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream);
+}
+// After a copy from the caller's buffer: pageable memory is staged already, pinned
+// memory is read by the device until the copy is done.
+cudaError_t caller_buffer_free(SorsHandle* h, const void* src) {
+    cudaPointerAttributes at;
+    const cudaError_t e = cudaPointerGetAttributes(&at, src);
+    if (e == cudaSuccess && at.type == cudaMemoryTypeUnregistered) return cudaSuccess;
+    if (e != cudaSuccess) cudaGetLastError();
+    return cudaStreamSynchronize(h->stream);
+}
 cudaError_t d2h(SorsHandle* h, void* dst, const void* src, size_t bytes) {
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream);
     return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
@@ -479,7 +493,11 @@ int build_tet_chunks(SorsHandle* h, const int32_t* conn, const double* X, const 
     if (h->nv != 4 || !(h->s.material == 0 || h->s.material == 2) || h->N == 0) return SORS_OK;
     const int N = h->N, E = h->E;
     const int hsz = mixed(h) ? 4 : 8;
-    const ChunkLimits lim = chunk_limits(hsz, h->s.material);
+    ChunkLimits lim = chunk_limits(hsz, h->s.material);
+    // small meshes: chunks for two blocks on every SM rather than full ones (each costs a
+    // latency per round of its 256 threads, and the shared elements' second evaluation
+    // runs on SMs that would idle)
+    lim.rows = std::min(lim.rows, std::max(8, (N + 2 * kResidentMaxBlocks - 1) / (2 * kResidentMaxBlocks)));
     // two blocks per SM must fit (227 KB of shared memory per SM)
     if (chunk_smem_bytes(hsz, h->s.material, h->max_pairs) > 113 * 1024) return SORS_OK;
     for (int i = 0; i < N; i++) {
@@ -1887,6 +1905,20 @@ int minimize(SorsHandle* h, double dt, SorsStepStats* stats) {
         prev_g = gn;
         prev_eta = eta;
         int pit = 0;
+        if (!ahead && probe && m == 0 && h->batch.nmem <= 1 && h->s.linear_solver == 0 &&
+            !(h->s.project_spd == 2 && h->s.newton_safeguard)) {
+            // the probed gradient is on the host: solve and update, then one read
+            h->tl_active = false;
+            if ((st = pcg_one_launch<VT>(h, eta, res_tol > 0.0 ? 0.1 * res_tol : 0.0, nullptr, nullptr, &ahead,
+                                         &refreshed)))
+                return st;
+            if (ahead) {
+                launch_newton_update<VT>(n, (const VT*)h->x, 1.0, h->q, h->q, h->partials, h->sc, 6, h->stream,
+                                         h->s.project_spd == 2 && !h->proj_fallback ? 2 : 1);
+                CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
+                CK(cudaStreamSynchronize(h->stream));
+            }
+        }
         if (ahead) {
             if ((st = pcg_one_launch_done<VT>(h, refreshed, &pit))) return st;
         } else if ((st = newton_solve<HT, VT>(h, dt, eta, res_tol > 0.0 ? 0.1 * res_tol : 0.0, &pit))) {
@@ -2494,7 +2526,7 @@ int minimize_sqp(SorsHandle* h, double dt, SorsStepStats* stats) {
     std::vector<double> xpair(6 * (size_t)np), mu_pair;
     PairRows R;
     h->md_work.assign(np, 0);
-    if (m) CK(h2d(h, h->cnode_d, cnode.data(), sizeof(int) * m));
+    if (m) CK(h2d_staged(h, h->cnode_d, cnode.data(), sizeof(int) * m));
     std::vector<char> inW(m, 0);
     std::vector<double> b(m), xc(3 * (size_t)m), chk(2 * (size_t)m);
     std::vector<double4> cnb(m);
@@ -2518,9 +2550,9 @@ int minimize_sqp(SorsHandle* h, double dt, SorsStepStats* stats) {
         double abs_tol = 0.0;   // set by the first (cold) solve of this iteration
         if ((st = eval_system<HT>(h, dt, true, kAsmFull))) return st;
         launch_gather_nodes(m, h->cnode_d, h->q, h->cpos_d, h->stream);
-        if (m) CK(d2h(h, xc.data(), h->cpos_d, sizeof(double) * 3 * m));
         CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        if (m) CK(d2h(h, xc.data(), h->cpos_d, sizeof(double) * 3 * m));
+        else CK(cudaStreamSynchronize(h->stream));
         if (h->sc_host->status & kFlagInverted) return fail(SORS_ERR_INVERTED, "Inverted Elements");
         for (int c = 0; c < m; c++) {
             const double* nn = &cn[3 * (size_t)c];
@@ -2529,7 +2561,7 @@ int minimize_sqp(SorsHandle* h, double dt, SorsStepStats* stats) {
             cnb[c] = make_double4(nn[0], nn[1], nn[2], b[c]);
             if (it == 0) inW[c] = b[c] > 0.0;  // start with the constraints violated now
         }
-        if (m) CK(h2d(h, h->cnb_d, cnb.data(), sizeof(double4) * m));
+        if (m) CK(h2d_staged(h, h->cnb_d, cnb.data(), sizeof(double4) * m));
         if (np) {
             launch_gather_nodes(2 * np, h->md_nodes_d, h->q, h->md_pos_d, h->stream);
             CK(d2h(h, xpair.data(), h->md_pos_d, sizeof(double) * 6 * np));
@@ -2546,8 +2578,9 @@ int minimize_sqp(SorsHandle* h, double dt, SorsStepStats* stats) {
                 h->pflag_h[v] = (uint8_t)((h->pflag_h[v] & 7u) | (inW[c] ? 8u : 0u));
                 h->pn_h[v] = cnb[c];
             }
-            CK(h2d(h, h->pflag_d, h->pflag_h.data(), (size_t)N));
-            if (m) CK(h2d(h, h->pn_d, h->pn_h.data(), sizeof(double4) * N));
+            CK(h2d_staged(h, h->pflag_d, h->pflag_h.data(), (size_t)N));
+            // the normals and bounds of this linearisation: unchanged by the working set
+            if (m && inner_used == 1) CK(h2d_staged(h, h->pn_d, h->pn_h.data(), sizeof(double4) * N));
             // particular solution: the constraints alone on the first solve, the
             // previous step with the new working set imposed on re-solves
             if (inner == 0) launch_qp_x0(N, h->pflag_d, h->pn_d, h->q, h->qPrev, h->mval, dt, h->qp_x0, h->stream);
@@ -2731,8 +2764,7 @@ int step_resident(SorsHandle* h, double dt, int substeps, SorsStepStats* stats) 
                             h->stream);
         if (stats) stats->substeps++;
     }
-    CK(cudaStreamSynchronize(h->stream));
-    CK(cudaGetLastError());
+    CK(cudaGetLastError());  // the callers synchronise after copying the result
     return SORS_OK;
 }
 
@@ -3263,7 +3295,7 @@ int sors_set_initial_deformation(SorsHandle* h, const double* q) {
     int st;
     if ((st = set_device(h))) return st;
     if ((st = dof_in(h, h->qPrev, q, cudaMemcpyHostToDevice))) return st;
-    CK(cudaStreamSynchronize(h->stream));
+    CK(caller_buffer_free(h, q));
     return SORS_OK;
 }
 
@@ -3272,7 +3304,7 @@ int sors_set_initial_velocity(SorsHandle* h, const double* v) {
     int st;
     if ((st = set_device(h))) return st;
     if ((st = dof_in(h, h->vPrev, v, cudaMemcpyHostToDevice))) return st;
-    CK(cudaStreamSynchronize(h->stream));
+    CK(caller_buffer_free(h, v));
     return SORS_OK;
 }
 
