@@ -79,6 +79,7 @@ struct Scratch {
     u64 bar[4];                    // cluster form: one mbarrier per site
     double part[kWarps][8];        // warps' partial values
     double tot[2];
+    double irz;                    // 1 / r.z
     double zc[6][2];               // the range's coarse correction, two partial sums each
     int abort, pad;
     double slot[kVals][16];  // cluster form: the blocks' messages, by value

@@ -76,7 +76,7 @@ __host__ __device__ inline Off offsets(const ResidentPlan& pl) {
     o.sov = at; at = up(at + (pl.max_rows + 1) * 4);
     o.sgb = at; at = up(at + pl.max_rows * 4);
     o.shalo = at; at = up(at + (pl.cluster ? 0 : pl.max_halo * 4));
-    o.spp = at; at = up(at + (pl.cluster ? (pl.max_rows + 1) * 4 : 0));
+    o.spp = at; at = up(at + (pl.cluster ? pl.max_push * 2 : 0));
     o.spush = at; at = up(at + (pl.cluster ? pl.max_push * 4 : 0));
     o.scol = at; at = up(at + pl.max_over * 2);
     o.sval = at;
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
     int* sov = reinterpret_cast<int*>(smem + o.sov);
     int* sgb = reinterpret_cast<int*>(smem + o.sgb);
     int* shalo = reinterpret_cast<int*>(smem + o.shalo);
-    int* spp = reinterpret_cast<int*>(smem + o.spp);
+    uint16_t* spp = reinterpret_cast<uint16_t*>(smem + o.spp);
     int* spush = reinterpret_cast<int*>(smem + o.spush);
     uint16_t* scol = reinterpret_cast<uint16_t*>(smem + o.scol);
     VT* sval = reinterpret_cast<VT*>(smem + o.sval);
@@ -157,10 +157,13 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
         for (int k = lane; k < n; k += 32) scol[sov[i] + k] = pl.lcol[gb + k];
         for (int k = lane; k < 9 * nres; k += 32) sval[9 * sov[i] + k] = __ldg(a.H + 9 * (size_t)gb + k);
     }
+    int np = 0;  // border z to push: row spp, to spush
     if constexpr (CL) {
-        const int q0 = pl.push_ptr[r0], np = pl.push_ptr[r0 + nr] - q0;
-        for (int i = t; i <= nr; i += kT) spp[i] = pl.push_ptr[r0 + i] - q0;
+        const int q0 = pl.push_ptr[r0];
+        np = pl.push_ptr[r0 + nr] - q0;
         for (int k = t; k < np; k += kT) spush[k] = pl.push[q0 + k];
+        for (int i = t; i < nr; i += kT)
+            for (int k = pl.push_ptr[r0 + i] - q0; k < pl.push_ptr[r0 + i + 1] - q0; k++) spp[k] = (uint16_t)i;
     } else {
         for (int k = t; k < nh; k += kT) shalo[k] = pl.halo[h0 + k];
     }
@@ -233,18 +236,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
             project<VT>(pf, a.pn + row, z);
 #pragma unroll
             for (int k = 0; k < 3; k++) zs[k] = z[k];
-            if constexpr (CL) {
-                for (int k = spp[t]; k < spp[t + 1]; k++) {
-                    const int d = spush[k];
-                    const unsigned dst = remote(sz + 4 * (d & 0xffff), d >> 16), rb = remote(&sh->bar[1], d >> 16);
-                    if constexpr (sizeof(VT) == 4) {
-                        push(dst, rb, z[0], z[1], z[2]);
-                    } else {
-                        push(dst, rb, z[0], z[1]);
-                        push(dst + 16, rb, z[2]);
-                    }
-                }
-            } else {
+            if constexpr (!CL) {
                 u64 w[Z];
                 if constexpr (sizeof(VT) == 4) {
 #pragma unroll
@@ -262,6 +254,22 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
                 acc[0] += (double)r[k] * (double)z[k];
                 acc[1] += (double)r[k] * (double)r[k];
             }
+        }
+        if constexpr (CL) {
+            // a thread per push (a row may have several readers)
+            __syncthreads();
+            for (int k = t; k < np; k += kT) {
+                const int d = spush[k];
+                const VT* z = reinterpret_cast<const VT*>(smem + o.sx) + 9 * (int)spp[k] + 6;
+                const unsigned dst = remote(sz + 4 * (d & 0xffff), d >> 16), rb = remote(&sh->bar[1], d >> 16);
+                if constexpr (sizeof(VT) == 4) {
+                    push(dst, rb, z[0], z[1], z[2]);
+                } else {
+                    push(dst, rb, z[0], z[1]);
+                    push(dst + 16, rb, z[2]);
+                }
+            }
+            __syncwarp();
         }
         if ((t & ~31) < nr) {  // a warp with rows
 #pragma unroll
@@ -376,6 +384,9 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
         // and a warp in pieces runs what follows once per piece
         __syncwarp();
         __syncthreads();
+        // the coming beta's divisor, on a warp that has time: every thread has read the
+        // last one before this barrier and reads this one after the sums' barriers
+        if (t == kT - 1) sh->irz = 1.0 / rz;
         double pqw = 0.0, yw[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         for (int base = 0; base + (t & ~31) / LPR < nr; base += NG) {
             const int i = base + g;
@@ -472,7 +483,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
         ok = exchange<1, 2, 2, CL>(acc, sh, G, ++epoch, a.box, par1, nh * kZBytes, nullptr);
         par1 ^= 1u;
         if (!ok) break;
-        beta = acc[0] / rz;
+        beta = acc[0] * sh->irz;
         rz = acc[0];
         rr = acc[1];
         it++;
