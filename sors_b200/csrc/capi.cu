@@ -1075,12 +1075,17 @@ void choose_parts(SorsHandle* h) {
         h->parts_G = std::max(1, std::min(16, (N + 31) / 32));
         return;
     }
-    // Grid: 64 blocks, more where a block's rows would not have a lane group each.
-    // A sum over 148 blocks takes 2.2 us, over 64 1.4 us; 4,225 FP64 nodes per
-    // step: 148 blocks 5.6 ms, 96 5.0, 64 5.1, 36 5.4; 10,648 FP32 nodes per three
-    // steps: 148 blocks 48 ms, 96 44, 64 41, 36 50.
-    const int per = hs == 4 ? 160 : 128;
-    const int G = std::max(1, std::min({gmax, (N + 15) / 16, std::max(64, (N + per - 1) / per)}));
+    // Grid: more blocks take fewer iterations (more, smaller aggregates) and longer
+    // sums (over 148 blocks 2.2 us, over 64 1.4 us).  ms by number of blocks, 64 / 80 /
+    // 96 / 128 / 148: a step of 4,225 FP64 nodes 1.46 / 1.34 / 1.35 / 1.37 / 1.48, of
+    // 9,856 FP32 nodes 1.85 / 1.80 / 1.77 / 1.83 / 1.95; three SQP steps of 10,648 FP32
+    // nodes 12.2 / 12.9 / 12.2 / 13.7 / 14.5 (67: 13.4); an adjoint of 3,321 FP64 hex
+    // nodes 32.7 / 33.4 / 34.0 / 37.1 / 39.2.  Counts with many halvings bisect best.
+    const int per = hs == 4 ? 160 : 128;  // rows that have a lane group each
+    int G = gmax;
+    for (int g : {64, 96, 128})
+        if (g < G && N <= g * per && (g > 64 || N < 4000)) G = g;
+    G = std::max(1, std::min(G, (N + 15) / 16));
     if (N <= G * (kResidentThreads - 16) && bytes <= G * 300 * 1024.0) {
         h->parts_form = 2;
         h->parts_G = G;
