@@ -71,7 +71,10 @@ typedef struct SorsSettings {
                                 plus an exact coarse correction on per-aggregate
                                 rigid-body modes (no reference counterpart);
                                 0: block Jacobi; 2 (default): 1 for meshes of
-                                20,000 nodes or more                              */
+                                20,000 nodes or more.  Where a whole solve is one
+                                launch (up to some 300,000 nodes) the correction
+                                costs no exchange of its own and 2 means 1 at
+                                every size; it changes iterates, not solutions    */
     int32_t linear_solver;   /* Newton systems of "minimize_newton": 0 (default)
                                 PCG; 1 MINRES, which takes the Newton step of an
                                 indefinite exact Hessian as the reference's LDL^T

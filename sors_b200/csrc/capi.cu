@@ -1288,7 +1288,7 @@ int ensure_stream(SorsHandle* h) {
     pl.G = h->parts_G;
     pl.A = h->parts_A;
     pl.N = N;
-    const int gr = 32 / pl.lpr;
+    const int gr = 32 / kStreamLanes;
     const int nagg = pl.A * pl.G, G = pl.G;
     pl.nc = 6 * nagg;
     const int w16 = 16 / hs;

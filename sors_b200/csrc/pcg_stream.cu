@@ -1,19 +1,21 @@
 // pcg_stream.cu -- a whole two-level PCG solve in one launch for meshes whose
 // matrix does not fit on the SMs: the matrix streams through shared memory.
 //
-// An iteration as separate launches (p, SpMV, update with restriction, coarse
-// solve with prolongation) took 103 us on the 3.0M-tet block, 66 us of it the
-// SpMV at 0.75 of the measured copy bandwidth: nine strided 8-byte loads per
-// lane touch every line nine times, so the L1 tags, not HBM, bound it, and p
-// came through the same path.  On meshes whose matrix stays in L2 (100,000
-// nodes, 52 MB in FP32) the launches and their reductions were most of it.
+// Between the meshes whose matrix the SMs hold and those whose matrix HBM bounds,
+// an iteration as separate launches (p, SpMV, update with restriction, coarse
+// solve with prolongation) is bound by launches, cold starts and reductions, the
+// matrix (52 MB of FP32 at 100,000 nodes) staying in L2.  A step, launches ->
+// here: 77,841 FP32 nodes 11.2 -> 6.7 ms, 169,781 17.5 -> 12.9, FP64 24.1 -> 16.5,
+// 291,870 25.3 -> 19.8; at 522,801 nodes, where HBM bounds both, 36.7 and 37.1.
+// What bounds it now: the shared-memory wavefronts of the product (a block's nine
+// values 2-way conflicting, p gathered: 30 per 32 blocks) and the sums' round trips.
 //
 // Here one block per SM owns a contiguous range of rows for the whole solve:
-//   matrix   each warp takes every 16th group of four rows; the group's CSR
-//            blocks are contiguous, so one thread fetches them (and their column
-//            indices, and the rows' offsets) with bulk copies (TMA) into the
-//            warp's ring of two to four groups, and the warp multiplies from
-//            shared memory.  No load instruction of the product goes to global
+//   matrix   each warp takes every 16th group of eight rows (four lanes a row);
+//            the group's CSR blocks are contiguous, so one thread fetches them
+//            (and their column indices, and the rows' offsets) with bulk copies
+//            (TMA) into the warp's ring of up to four groups, and the warp
+//            multiplies from shared memory.  No load instruction of the product goes to global
 //            memory; nothing waits for another warp.
 //   p        the range's own and border columns in shared memory (p = z + beta p
 //            formed by every range that reads it, from the same z)
@@ -36,7 +38,8 @@ namespace sors {
 
 namespace {
 
-constexpr int kMaxA = kStreamMaxAgg;
+constexpr int kMaxA = kStreamMaxAgg, kLPR = kStreamLanes;
+constexpr int kGR = 32 / kLPR;  // rows per group
 
 struct SOff {
     int zc, part, y, a, sp, srp, halo, bar, ring;
@@ -78,10 +81,9 @@ __device__ __forceinline__ void bulk(unsigned dst, const void* src, unsigned byt
                  : "memory");
 }
 
-template <typename VT, int kLPR>
+template <typename VT>
 __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<VT> a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int kGR = 32 / kLPR;  // rows per group
     constexpr int P = Lay<VT>::P, Z = Lay<VT>::Z;
     constexpr int BB = 9 * (int)sizeof(VT);  // bytes of a matrix block
     double eta2, abs_tol2;
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
         clear_part();
         __syncwarp();
         __syncthreads();
-        // q = A p: a group of eight lanes per row, four rows at a time
+        // q = A p
         double pqw = 0.0, yw[6] = {0, 0, 0, 0, 0, 0};
         int ag = 0;
         int slot = 0;
@@ -537,9 +539,9 @@ size_t stream_smem(const StreamPlan& pl, int vsize) {
     return (size_t)at + (size_t)kWarps * pl.depth * pl.group_bytes;
 }
 
-template <typename VT, int LPR>
-static int launch_one(const StreamPlan& pl, const StreamArgs<VT>& a, cudaStream_t st) {
-    auto kern = k_pcg_stream<VT, LPR>;
+template <typename VT>
+int launch_pcg_stream(const StreamPlan& pl, const StreamArgs<VT>& a, cudaStream_t st) {
+    auto kern = k_pcg_stream<VT>;
     static std::atomic<int> done[kMaxDevices];
     int dev = 0;
     cudaGetDevice(&dev);
@@ -562,11 +564,6 @@ static int launch_one(const StreamPlan& pl, const StreamArgs<VT>& a, cudaStream_
     if (e != cudaSuccess) return (int)e;
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     return 0;
-}
-template <typename VT>
-int launch_pcg_stream(const StreamPlan& pl, const StreamArgs<VT>& a, cudaStream_t st) {
-    if (pl.lpr == 2) return launch_one<VT, 2>(pl, a, st);
-    return pl.lpr == 4 ? launch_one<VT, 4>(pl, a, st) : launch_one<VT, 8>(pl, a, st);
 }
 template int launch_pcg_stream<float>(const StreamPlan&, const StreamArgs<float>&, cudaStream_t);
 template int launch_pcg_stream<double>(const StreamPlan&, const StreamArgs<double>&, cudaStream_t);

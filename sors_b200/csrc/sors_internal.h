@@ -243,13 +243,13 @@ struct ResidentArgs {
 // A whole two-level PCG solve in one launch with the matrix streaming through
 // shared memory (pcg_stream.cu): G blocks, block b owning the rows [row0[b],
 // row0[b + 1]), A aggregates of agg_rows[b] consecutive rows each.
-constexpr int kStreamMaxAgg = 4;
+constexpr int kStreamMaxAgg = 2;  // aggregates per row range
+constexpr int kStreamLanes = 4;   // lanes per row
 struct StreamPlan {
     int G = 0, A = 1, N = 0;
-    int lpr = 4;                        // lanes per row
     int nc = 0, ld = 0;                 // coarse unknowns 6 A G, leading dimension of their inverse
     int max_rows = 0, max_cols = 0, max_halo = 0;
-    int group_bytes = 0, depth = 2;     // ring slot: four rows' matrix blocks, column indices, offsets; slots per warp
+    int group_bytes = 0, depth = 2;     // ring slot: a group's matrix blocks, column indices, offsets; slots per warp
     int slot_col = 0, slot_off = 0;     // byte offsets in a slot
     int a_shared = 0;                   // the block's rows of the coarse inverse are kept in shared memory
     int evict_first = 0;                // the matrix does not fit in L2

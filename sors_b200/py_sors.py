@@ -60,7 +60,7 @@ class SimulationSettings:
         self.maxBlocksPerKernel = 0        # grid cap per kernel (0: whole GPU)
         self.newtonSafeguard = False       # halve Newton steps that raise ||g|| (adaptive Hessian only)
         # block Jacobi + coarse rigid-body correction: True, False or "auto"
-        # (on for meshes of 20,000 nodes or more)
+        # (on for meshes of 20,000 nodes or more, and wherever a solve is one launch)
         self.twoLevelPreconditioner = "auto"
         # Newton linear solver of "minimize_newton": "pcg", or "minres" for the
         # exact Newton step of an indefinite Hessian (the reference's LDL^T step)
