@@ -2847,20 +2847,22 @@ void locality_order(SorsHandle* h, int N, int E, int nv, const double* X, const 
 // parts), 123k tets 249 -> 188 (148), a hex arm 362 -> 279 (148).
 void number_by_parts(SorsHandle* h, const double* X, std::vector<int>& n2o) {
     const int N = h->N, G = h->parts_G, A = h->parts_A;
+    // the nodes, with their coordinates beside them, are moved: a cut reads in order
+    struct Pt { double x[3]; int i; };
+    std::vector<Pt> pt(N);
+    for (int i = 0; i < N; i++) pt[i] = {{X[3 * (size_t)i], X[3 * (size_t)i + 1], X[3 * (size_t)i + 2]}, i};
     n2o.resize(N);
-    for (int i = 0; i < N; i++) n2o[i] = i;
     h->part0.assign((size_t)G * A + 1, N);
     double lo[3], hi[3];
-    auto extent = [&](const int* a, const int* b, double* l, double* u) {
+    auto extent = [&](const Pt* a, const Pt* b, double* l, double* u) {
         for (int k = 0; k < 3; k++) { l[k] = 1e300; u[k] = -1e300; }
         for (; a < b; a++)
             for (int k = 0; k < 3; k++) {
-                const double x = X[3 * (size_t)*a + k];
-                l[k] = std::min(l[k], x);
-                u[k] = std::max(u[k], x);
+                l[k] = std::min(l[k], a->x[k]);
+                u[k] = std::max(u[k], a->x[k]);
             }
     };
-    extent(n2o.data(), n2o.data() + N, lo, hi);
+    extent(pt.data(), pt.data() + N, lo, hi);
     const double ext = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
     auto spread = [](uint64_t v) {
         v &= 0x1fffff;
@@ -2881,22 +2883,22 @@ void number_by_parts(SorsHandle* h, const double* X, std::vector<int>& n2o) {
             }
         }
     });
-    // nodes [a, b) of n2o into `parts` parts; the first half's size from `head`
+    // the lower m - a of the nodes [a, b) along their longest extent go first
     auto split = [&](int a, int b, int m) {
         double l[3], u[3];
-        extent(n2o.data() + a, n2o.data() + b, l, u);
+        extent(pt.data() + a, pt.data() + b, l, u);
         int ax = 0;
         for (int k = 1; k < 3; k++)
             if (u[k] - l[k] > u[ax] - l[ax]) ax = k;
-        std::nth_element(n2o.begin() + a, n2o.begin() + m, n2o.begin() + b, [&](int p, int q) {
-            const double x = X[3 * (size_t)p + ax], y = X[3 * (size_t)q + ax];
-            return x < y || (x == y && p < q);
+        std::nth_element(pt.begin() + a, pt.begin() + m, pt.begin() + b, [ax](const Pt& p, const Pt& q) {
+            return p.x[ax] < q.x[ax] || (p.x[ax] == q.x[ax] && p.i < q.i);
         });
     };
     // aggregates of a range: whole warps of rows each
     std::function<void(int, int, int, int, int)> leaves = [&](int a, int b, int k0, int k1, int L) {
         if (k1 - k0 == 1) {
             h->part0[k0] = a;
+            for (int k = a; k < b; k++) n2o[k] = pt[k].i;
             std::sort(n2o.begin() + a, n2o.begin() + b,
                       [&](int p, int q) { return code[p] < code[q] || (code[p] == code[q] && p < q); });
             return;
@@ -2913,7 +2915,7 @@ void number_by_parts(SorsHandle* h, const double* X, std::vector<int>& n2o) {
         }
         const int half = (g1 - g0) / 2, m = a + (int)((int64_t)(b - a) * half / (g1 - g0));
         if (m > a && m < b) split(a, b, m);
-        if (depth < 3 && b - a > 20000) {
+        if (depth < 3 && b - a > 4000) {
             std::thread t([&]() { ranges(a, m, g0, g0 + half, depth + 1); });
             ranges(m, b, g0 + half, g1, depth + 1);
             t.join();
