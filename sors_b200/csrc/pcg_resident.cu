@@ -35,12 +35,16 @@
 //
 // All sums run in a fixed order, so a solve is bit-reproducible.
 //
-// Measured, whole iteration (three launches before -> here): cluster, 1,728
-// FP32 nodes 15 -> 3.8 us; grid, 4,225 FP64 nodes 15 -> 6.4 us, 10,648 FP32 nodes
-// 17 -> 6.2 us, 18,921 FP64 hex nodes (33 MB of matrix) 25 -> 10.8 us.  What bounds
-// it now: the two sums' round trips through L2 (1.4 us each over 64 blocks, of
-// which 1.2 us is one store and one load) or, in a cluster, latency of the
-// dependent FP64 steps (about 1,000 cycles a sum, 1,100 a product).
+// Measured, whole iteration with block Jacobi (three launches before -> here):
+// cluster, 1,728 FP32 nodes 15 -> 3.8 us; grid, 4,225 FP64 nodes 15 -> 6.4 us,
+// 10,648 FP32 nodes 17 -> 6.2 us, 18,921 FP64 hex nodes (33 MB of matrix) 25 -> 10.8
+// us.  With the two-level preconditioner, which takes two to five times fewer
+// iterations, and a solve's loading shared out over them: cluster, 525 FP64 nodes
+// 4.0 us; grid, 4,225 FP64 nodes 8.4, 9,856 FP32 nodes 9.8, 22,680 FP64 nodes 14.7,
+// the hexes 14.6 us.  What bounds it now: the two sums' round trips through L2
+// (1.4 us each over 64 blocks, 2.2 over 148, of which 1.2 us is one store and one
+// load) or, in a cluster, latency of the dependent FP64 steps (about 1,000 cycles a
+// sum, 1,100 a product).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
