@@ -1494,7 +1494,12 @@ int pcg_one_launch(SorsHandle* h, double eta, double abs_tol, const double* g, c
 // After a one-launch solve, its scalars in sc_host.
 template <typename VT>
 int pcg_one_launch_done(SorsHandle* h, bool refreshed, int* iters) {
-    if (h->sc_host->status & kFlagTimeout) return fail(SORS_ERR_CUDA, "the PCG blocks did not meet within the limit");
+    if (h->sc_host->status & kFlagTimeout) {
+        // blocks left the exchange at different epochs: the next solve starts from empty mailboxes
+        CK(cudaMemsetAsync(h->res_zg, 0, (size_t)((char*)h->res_epoch - (char*)h->res_zg) + 256, h->stream));
+        CK(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
+        return fail(SORS_ERR_CUDA, "the PCG blocks did not meet within the limit");
+    }
     if (h->res_state == 1 ? h->res.coarse != 0 : true)
         coarse_rate_check(h, refreshed, &h->rc_ref_rate, &h->rc_ready);
     *iters = h->sc_host->it;
