@@ -1024,6 +1024,16 @@ void coarse_rate_check(SorsHandle* h, bool refreshed, double* ref_rate, bool* re
     }
 }
 
+// A coarse operator built for the last solve (refreshed) is not kept when the
+// Hessian turns out to hold inverted elements or NaN: the one-launch PCG builds it
+// before the host has read the evaluation's scalars.
+void coarse_state_check(SorsHandle* h, bool refreshed, bool* ready) {
+    const DevScalars& sh = *h->sc_host;
+    if (refreshed && ((sh.status & kFlagInverted) || !(sh.gnorm2 == sh.gnorm2) || !(sh.rr == sh.rr) ||
+                      !(sh.rz == sh.rz) || !(sh.pq == sh.pq)))
+        *ready = false;
+}
+
 // Aggregate pairs and their Hessian blocks (counting sort by pair key): pair k
 // holds items [pair_ptr[k], pair_ptr[k + 1]), each (CSR block, its row).
 void coarse_pairs(const SorsHandle* h, const std::vector<int>& aid, int nagg, std::vector<int>& pair_ptr,
@@ -1500,8 +1510,10 @@ int pcg_one_launch_done(SorsHandle* h, bool refreshed, int* iters) {
         CK(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
         return fail(SORS_ERR_CUDA, "the PCG blocks did not meet within the limit");
     }
-    if (h->res_state == 1 ? h->res.coarse != 0 : true)
+    if (h->res_state == 1 ? h->res.coarse != 0 : true) {
         coarse_rate_check(h, refreshed, &h->rc_ref_rate, &h->rc_ready);
+        coarse_state_check(h, refreshed, &h->rc_ready);
+    }
     *iters = h->sc_host->it;
     if (!h->sc_host->breakdown) return SORS_OK;
     int st = record_curvature<VT>(h);
@@ -1563,7 +1575,10 @@ int pcg_solve(SorsHandle* h, double eta, double abs_tol, int* iters, const doubl
         if (st) return st;
     }
     // loose solves converge faster per decade and are not counted
-    if (h->tl_active) coarse_rate_check(h, refreshed, &h->tl_ref_rate, &h->tl_ready);
+    if (h->tl_active) {
+        coarse_rate_check(h, refreshed, &h->tl_ref_rate, &h->tl_ready);
+        coarse_state_check(h, refreshed, &h->tl_ready);
+    }
     if (h->sc_host->breakdown && h->sc_host->it == 0 && !(h->s.project_spd == 2 && !h->proj_fallback))
         return fail(SORS_ERR_PCG_BREAKDOWN, "PCG breakdown: the Hessian is not positive definite");
     return SORS_OK;
@@ -1897,6 +1912,7 @@ int minimize(SorsHandle* h, double dt, SorsStepStats* stats) {
         }
         CK(cudaMemcpyAsync(h->sc_host, h->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
+        if (ahead) coarse_state_check(h, refreshed, &h->rc_ready);
         if (h->sc_host->status & kFlagInverted)
             return fail(SORS_ERR_INVERTED, "Inverted Elements");
         double gn = sqrt(h->sc_host->gnorm2);
