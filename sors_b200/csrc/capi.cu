@@ -1060,30 +1060,32 @@ void coarse_pairs(const SorsHandle* h, const std::vector<int>& aid, int nagg, st
             items[(size_t)keypos[(size_t)aid[i] * nagg + aid[h->col_h[b]]]++] = make_int2(b, i);
 }
 
-// The form of the one-launch PCG and its number of row ranges, from the mesh's
-// size (before the pattern is built: tets have about 3 N + 2 E blocks, hexes N + 26 E):
-// 1 one cluster, 2 a grid with the matrix on the SMs, 3 a grid with a streamed matrix.
-void choose_parts(SorsHandle* h) {
-    const int N = h->N;
-    const size_t hs = hsize(h);
-    const double blocks = h->nv == 4 ? 3.0 * N + 2.0 * h->E : N + 26.0 * h->E, bytes = blocks * 9 * hs;
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) sms = 0;
+// The form of the one-launch PCG and its row ranges, from the mesh's size (before
+// the pattern is built: tets have about 3 N + 2 E blocks, hexes N + 26 E): form 1 one
+// cluster, 2 a grid with the matrix on the SMs, 3 a grid with a streamed matrix, 0
+// none; G ranges of A aggregates.
+struct Parts {
+    int form = 0, G = 0, A = 1;
+};
+Parts pick_parts(int N, int E, int nv, size_t hs, int sms, int max_blocks, bool two_level) {
+    Parts p;
+    const double blocks = nv == 4 ? 3.0 * N + 2.0 * E : N + 26.0 * E, bytes = blocks * 9 * hs;
     // a handle whose grids are capped takes the same share of the SMs
     int gmax = std::min(sms, kResidentMaxBlocks);
-    if (h->s.max_blocks > 0) gmax = std::min(gmax, std::max(1, h->s.max_blocks * kResidentMaxBlocks / kRedBlocks));
-    if (gmax < 1) return;
+    if (max_blocks > 0) gmax = std::min(gmax, std::max(1, max_blocks * kResidentMaxBlocks / kRedBlocks));
+    if (gmax < 1) return p;
     // One cluster up to 3.3 MB of matrix: its exchanges are three times cheaper,
     // but 16 SMs hold and multiply the whole matrix.  Measured per iteration
     // (cluster / grid): FP32 tets 2,744 nodes 3.7 / 5.3 us, 6,859 nodes (3.5 MB)
     // 5.8 / 6.2 us; FP64 tets 1,000 nodes 4.0 / 6.2 us, 3,375 nodes (3.4 MB) 6.3 /
     // 6.5 us, 4,225 nodes 7.6 / 6.5 us; FP64 hexes 891 nodes 13.6 / 18.1 us per
-    // adjoint iteration, 2,025 nodes 18.2 / 19.4 us.
-    h->parts_A = 1;
-    if (N <= 16 * kResidentThreads && bytes <= 16 * 200 * 1024.0) {
-        h->parts_form = 1;
-        h->parts_G = std::max(1, std::min(16, (N + 31) / 32));
-        return;
+    // adjoint iteration, 2,025 nodes 18.2 / 19.4 us.  A cap below 16 blocks holds for
+    // it too: no kernel's grid is larger than the settings say.
+    const int C = max_blocks > 0 ? std::min(16, max_blocks) : 16;
+    if (N <= C * kResidentThreads && bytes <= C * 200 * 1024.0) {
+        p.form = 1;
+        p.G = std::max(1, std::min(C, (N + 31) / 32));
+        return p;
     }
     // Grid: more blocks take fewer iterations (more, smaller aggregates) and longer
     // sums (over 148 blocks 2.2 us, over 64 1.4 us).  ms by number of blocks, 64 / 80 /
@@ -1097,26 +1099,36 @@ void choose_parts(SorsHandle* h) {
         if (g < G && N <= g * per && (g > 64 || N < 4000)) G = g;
     G = std::max(1, std::min(G, (N + 15) / 16));
     if (N <= G * (kResidentThreads - 16) && bytes <= G * 300 * 1024.0) {
-        h->parts_form = 2;
-        h->parts_G = G;
-        return;
+        p.form = 2;
+        p.G = G;
+        return p;
     }
-    if (h->s.max_blocks > 0 || !h->s.two_level) return;
+    if (max_blocks > 0 || !two_level) return p;
     // Streamed: while the ranges' p, with their border columns, and the rings fit in
     // shared memory, and up to 2,500 rows a range (ms per step, launch per kernel /
     // streamed: 77,841 FP32 nodes 11.2 / 6.7, 169,781 17.5 / 12.9, FP64 24.1 / 16.5,
     // 291,870 25.3 / 19.8, 522,801 36.7 / 37.1).
     const double rows = (double)N / gmax, border = 7.0 * pow(rows, 2.0 / 3.0);
-    const double ring = 16.0 * 8.0 * (h->nv == 4 ? 16.0 : 27.0) * (9.0 * hs + 2.0);
+    const double ring = 16.0 * 8.0 * (nv == 4 ? 16.0 : 27.0) * (9.0 * hs + 2.0);
     if (rows > 2500.0 ||
         (rows + border) * (hs == 4 ? 16.0 : 24.0) + 4.0 * rows + 4.0 * border + 24e3 + ring > kResidentSmem)
-        return;
-    h->parts_form = 3;
-    h->parts_G = gmax;
+        return p;
+    p.form = 3;
+    p.G = gmax;
     // Aggregates per range: a second one takes a fifth off the iterations and adds
     // the matrix of four times the coarse unknowns to each (ms per step, 1 / 2 / 4:
     // 77,841 FP32 nodes 7.1 / 6.7 / 8.6, 169,781 14.2 / 12.9 / 14.2; 24,518: 4.3 / 4.5).
-    h->parts_A = rows < 400.0 ? 1 : 2;
+    p.A = rows < 400.0 ? 1 : 2;
+    return p;
+}
+
+void choose_parts(SorsHandle* h) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) sms = 0;
+    const Parts p = pick_parts(h->N, h->E, h->nv, hsize(h), sms, h->s.max_blocks, h->s.two_level != 0);
+    h->parts_form = p.form;
+    h->parts_G = p.G;
+    h->parts_A = p.A;
 }
 
 // Rows of each of a range's A aggregates (the last may have fewer): whole warps.
@@ -3181,6 +3193,13 @@ int sors_create(const double* X, int32_t n_nodes, const int32_t* conn, int32_t n
     CK(cudaStreamSynchronize(h->stream));
     *out = h;
     return SORS_OK;
+}
+
+// Not part of the ABI: pick_parts for the tests, out = {form, G, A}.
+void sors_pcg_parts(int32_t n_nodes, int32_t n_elems, int32_t nodes_per_elem, int32_t value_bytes, int32_t sms,
+                    int32_t max_blocks, int32_t two_level, int32_t* out) {
+    const Parts p = pick_parts(n_nodes, n_elems, nodes_per_elem, (size_t)value_bytes, sms, max_blocks, two_level != 0);
+    out[0] = p.form; out[1] = p.G; out[2] = p.A;
 }
 
 void sors_destroy(SorsHandle* h) {

@@ -1,0 +1,27 @@
+"""The rule that gives a mesh its one-launch PCG form and row ranges (host only)."""
+import ctypes as C
+
+import pytest
+
+
+def parts(n, e, nv=4, vsize=4, sms=148, cap=0, two_level=1):
+    from sors_b200 import _lib
+    fn = _lib.load().sors_pcg_parts
+    fn.restype = None
+    fn.argtypes = [C.c_int32] * 7 + [C.POINTER(C.c_int32)]
+    out = (C.c_int32 * 3)()
+    fn(n, e, nv, vsize, sms, cap, two_level, out)
+    return tuple(out)
+
+
+@pytest.mark.parametrize("n,e,nv", [(8, 5, 4), (525, 1536, 4), (2744, 13182, 4), (5000, 24000, 4), (891, 640, 8)])
+@pytest.mark.parametrize("vsize", [4, 8])
+@pytest.mark.parametrize("cap", [1, 2, 7, 8, 15, 16, 148])
+def test_grid_cap_holds_for_the_cluster(n, e, nv, vsize, cap):
+    """max_blocks is the largest grid of any kernel of the handle, below 16 blocks too."""
+    form, g, _ = parts(n, e, nv, vsize, cap=cap)
+    assert form == 0 or 1 <= g <= cap
+    if form:  # every range within a block's rows
+        assert n <= g * 512
+    if cap >= 16:
+        assert (form, g) == parts(n, e, nv, vsize)[:2] or form != 1
