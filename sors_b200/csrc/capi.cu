@@ -1072,7 +1072,8 @@ Parts pick_parts(int N, int E, int nv, size_t hs, int sms, int max_blocks, bool 
     const double blocks = nv == 4 ? 3.0 * N + 2.0 * E : N + 26.0 * E, bytes = blocks * 9 * hs;
     // a handle whose grids are capped takes the same share of the SMs
     int gmax = std::min(sms, kResidentMaxBlocks);
-    if (max_blocks > 0) gmax = std::min(gmax, std::max(1, max_blocks * kResidentMaxBlocks / kRedBlocks));
+    if (max_blocks > 0)
+        gmax = (int)std::min<long long>(gmax, std::max(1LL, (long long)max_blocks * kResidentMaxBlocks / kRedBlocks));
     if (gmax < 1) return p;
     // One cluster up to 3.3 MB of matrix: its exchanges are three times cheaper,
     // but 16 SMs hold and multiply the whole matrix.  Measured per iteration

@@ -25,3 +25,8 @@ def test_grid_cap_holds_for_the_cluster(n, e, nv, vsize, cap):
         assert n <= g * 512
     if cap >= 16:
         assert (form, g) == parts(n, e, nv, vsize)[:2] or form != 1
+
+
+@pytest.mark.parametrize("cap", [1184, 14_510_025, 2**31 - 1])
+def test_cap_above_the_whole_gpu_changes_nothing(cap):
+    assert parts(9856, 52488, cap=cap) == parts(9856, 52488)
