@@ -214,8 +214,8 @@ struct SorsHandle {
     // the numbering was not made by parts
     int parts_form = 0, parts_G = 0, parts_A = 1;
     std::vector<int> part0;
-    // one-launch PCG (ensure_resident): 0 not looked at, 1 planned, -1 not for this mesh
-    int res_state = 0;
+    // one-launch PCG (plan_one_launch): the matrix on the SMs (res) or streamed (str)
+    bool res_ready = false, str_ready = false;
     ResidentPlan res;
     unsigned long long *res_zg = nullptr, *res_box = nullptr;
     unsigned* res_epoch = nullptr;
@@ -225,9 +225,6 @@ struct SorsHandle {
     const int2* rc_ab = nullptr;
     const int* rc_row0 = nullptr;       // first row of each aggregate
     int rc_ld = 0;                      // leading dimension of rc_Ainv
-    // one-launch PCG with a streamed matrix (ensure_stream), for larger meshes: 0 not
-    // looked at, 1 planned, -1 not for this mesh
-    int str_state = 0;
     StreamPlan str;
     void* str_ws = nullptr;
     float4* str_woff = nullptr;
@@ -1063,11 +1060,12 @@ void coarse_pairs(const SorsHandle* h, const std::vector<int>& aid, int nagg, st
 // The form of the one-launch PCG and its row ranges, from the mesh's size (before
 // the pattern is built: tets have about 3 N + 2 E blocks, hexes N + 26 E): form 1 one
 // cluster, 2 a grid with the matrix on the SMs, 3 a grid with a streamed matrix, 0
-// none; G ranges of A aggregates.
+// none; G ranges of A aggregates.  after: only forms beyond this one (a plan that the
+// mesh's own rows and borders refuse).
 struct Parts {
     int form = 0, G = 0, A = 1;
 };
-Parts pick_parts(int N, int E, int nv, size_t hs, int sms, int max_blocks, bool two_level) {
+Parts pick_parts(int N, int E, int nv, size_t hs, int sms, int max_blocks, bool two_level, int after = 0) {
     Parts p;
     const double blocks = nv == 4 ? 3.0 * N + 2.0 * E : N + 26.0 * E, bytes = blocks * 9 * hs;
     // a handle whose grids are capped takes the same share of the SMs
@@ -1083,7 +1081,7 @@ Parts pick_parts(int N, int E, int nv, size_t hs, int sms, int max_blocks, bool 
     // adjoint iteration, 2,025 nodes 18.2 / 19.4 us.  A cap below 16 blocks holds for
     // it too: no kernel's grid is larger than the settings say.
     const int C = max_blocks > 0 ? std::min(16, max_blocks) : 16;
-    if (N <= C * kResidentThreads && bytes <= C * 200 * 1024.0) {
+    if (after < 1 && N <= C * kResidentThreads && bytes <= C * 200 * 1024.0) {
         p.form = 1;
         p.G = std::max(1, std::min(C, (N + 31) / 32));
         return p;
@@ -1099,12 +1097,12 @@ Parts pick_parts(int N, int E, int nv, size_t hs, int sms, int max_blocks, bool 
     for (int g : {64, 96, 128})
         if (g < G && N <= g * per && (g > 64 || N < 4000)) G = g;
     G = std::max(1, std::min(G, (N + 15) / 16));
-    if (N <= G * (kResidentThreads - 16) && bytes <= G * 300 * 1024.0) {
+    if (after < 2 && N <= G * (kResidentThreads - 16) && bytes <= G * 300 * 1024.0) {
         p.form = 2;
         p.G = G;
         return p;
     }
-    if (max_blocks > 0 || !two_level) return p;
+    if (after >= 3 || max_blocks > 0 || !two_level) return p;
     // Streamed: while the ranges' p, with their border columns, and the rings fit in
     // shared memory, and up to 2,500 rows a range (ms per step, launch per kernel /
     // streamed: 77,841 FP32 nodes 11.2 / 6.7, 169,781 17.5 / 12.9, FP64 24.1 / 16.5,
@@ -1123,10 +1121,10 @@ Parts pick_parts(int N, int E, int nv, size_t hs, int sms, int max_blocks, bool 
     return p;
 }
 
-void choose_parts(SorsHandle* h) {
+void choose_parts(SorsHandle* h, int after = 0) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) sms = 0;
-    const Parts p = pick_parts(h->N, h->E, h->nv, hsize(h), sms, h->s.max_blocks, h->s.two_level != 0);
+    const Parts p = pick_parts(h->N, h->E, h->nv, hsize(h), sms, h->s.max_blocks, h->tl_req != 0, after);
     h->parts_form = p.form;
     h->parts_G = p.G;
     h->parts_A = p.A;
@@ -1149,15 +1147,12 @@ std::vector<int> range_rows(const SorsHandle* h, int G, int A) {
     return row0;
 }
 
-// Plan of the one-launch PCG (pcg_resident.cu), made at the first solve that
-// could use it: the row ranges, their border columns and local column indices.
-int ensure_resident(SorsHandle* h) {
-    if (h->res_state != 0) return SORS_OK;
-    h->res_state = -1;
+// Plan of the one-launch PCG (pcg_resident.cu): the row ranges, their border columns
+// and local column indices.  res_ready stays false for a mesh it does not take.
+int plan_resident(SorsHandle* h) {
     const int N = h->N;
     const int hs = (int)hsize(h);
     ResidentPlan pl;
-    if (h->parts_form != 1 && h->parts_form != 2) return SORS_OK;
     pl.cluster = h->parts_form == 1;
     pl.G = h->parts_G;
     const std::vector<int> row0 = range_rows(h, pl.G, 1);
@@ -1295,18 +1290,14 @@ int ensure_resident(SorsHandle* h) {
     h->rcargs.N = N; h->rcargs.nagg = pl.G; h->rcargs.nc = nc;
     h->rcargs.fixed = h->node_mask; h->rcargs.off = pl.off;
     h->res = pl;
-    h->res_state = 1;
+    h->res_ready = true;
     return SORS_OK;
 }
 
-// Plan of the one-launch PCG with a streamed matrix (pcg_stream.cu), made at the
-// first solve of a mesh the resident form does not take.
-int ensure_stream(SorsHandle* h) {
-    if (h->str_state != 0) return SORS_OK;
-    h->str_state = -1;
+// Plan of the one-launch PCG with a streamed matrix (pcg_stream.cu).
+int plan_stream(SorsHandle* h) {
     const int N = h->N;
     const int hs = (int)hsize(h);
-    if (h->parts_form != 3) return SORS_OK;
     StreamPlan pl;
     pl.G = h->parts_G;
     pl.A = h->parts_A;
@@ -1454,7 +1445,21 @@ int ensure_stream(SorsHandle* h) {
     h->rcargs.N = N; h->rcargs.nagg = nagg; h->rcargs.nc = pl.nc;
     h->rcargs.fixed = h->node_mask; h->rcargs.off = pl.off;
     h->str = pl;
-    h->str_state = 1;
+    h->str_ready = true;
+    return SORS_OK;
+}
+
+// The plan of the handle's form, made at the first solve that could use it.  The form
+// was chosen by the mesh's size alone; one that its rows and borders refuse (a range of
+// many short rows, as of nodes without elements; borders of an unordered mesh) goes on
+// to the next, and past the last to the launches per kernel.
+int plan_one_launch(SorsHandle* h) {
+    while (h->parts_form && !h->res_ready && !h->str_ready) {
+        const int st = h->parts_form == 3 ? plan_stream(h) : plan_resident(h);
+        if (st) return st;
+        h->rc_ready = false;
+        if (!h->res_ready && !h->str_ready) choose_parts(h, h->parts_form);
+    }
     return SORS_OK;
 }
 
@@ -1480,37 +1485,42 @@ template <typename VT>
 int pcg_one_launch(SorsHandle* h, double eta, double abs_tol, const double* g, const NewtonForcing* nf, bool* ran,
                    bool* refreshed) {
     *ran = *refreshed = false;
-    int st = ensure_resident(h);
-    if (st) return st;
-    if (h->res_state != 1 && (st = ensure_stream(h))) return st;
-    if (h->res_state != 1 && h->str_state != 1) return SORS_OK;
-    const bool coarse = h->res_state == 1 ? h->res.coarse != 0 : true;
-    if (coarse && !h->rc_ready) {
-        if ((st = build_resident_coarse<VT>(h))) return st;
-        *refreshed = true;
+    while (!*ran) {
+        int st = plan_one_launch(h);
+        if (st) return st;
+        if (!h->parts_form) return SORS_OK;
+        const bool coarse = h->res_ready ? h->res.coarse != 0 : true;
+        if (coarse && !h->rc_ready) {
+            if ((st = build_resident_coarse<VT>(h))) return st;
+            *refreshed = true;
+        }
+        auto fill = [&](auto& a) {
+            a.row_ptr = h->row_ptr; a.diag_slot = h->diag_slot; a.H = (const VT*)h->H; a.g = g ? g : h->g;
+            a.x = (VT*)h->x; a.p0 = (VT*)h->p0; a.p1 = (VT*)h->p1; a.zg = h->res_zg; a.box = h->res_box;
+            a.eta2 = eta * eta; a.abs_tol2 = abs_tol * abs_tol; a.maxit = h->s.pcg_max_iter;
+            a.pflag = h->proj_flag; a.pn = h->proj_n; a.epoch = h->res_epoch; a.sc = h->sc;
+            a.fixed = h->node_mask;
+            a.Ainv = coarse ? (const VT*)h->rc_Ainv : nullptr;
+            if (nf) a.nf = *nf;
+        };
+        if (h->res_ready) {
+            ResidentArgs<VT> a;
+            fill(a);
+            *ran = launch_pcg_resident<VT>(h->res, a, h->stream) == 0;
+        } else {
+            StreamArgs<VT> a;
+            fill(a);
+            a.ws = (VT*)h->str_ws; a.woff = h->str_woff; a.board = h->str_board;
+            *ran = launch_pcg_stream<VT>(h->str, a, h->stream) == 0;
+        }
+        if (!*ran) {
+            // not on this device: the next form
+            cudaGetLastError();
+            *refreshed = false;
+            h->res_ready = h->str_ready = false;
+            choose_parts(h, h->parts_form);
+        }
     }
-    auto fill = [&](auto& a) {
-        a.row_ptr = h->row_ptr; a.diag_slot = h->diag_slot; a.H = (const VT*)h->H; a.g = g ? g : h->g;
-        a.x = (VT*)h->x; a.p0 = (VT*)h->p0; a.p1 = (VT*)h->p1; a.zg = h->res_zg; a.box = h->res_box;
-        a.eta2 = eta * eta; a.abs_tol2 = abs_tol * abs_tol; a.maxit = h->s.pcg_max_iter;
-        a.pflag = h->proj_flag; a.pn = h->proj_n; a.epoch = h->res_epoch; a.sc = h->sc;
-        a.fixed = h->node_mask;
-        a.Ainv = coarse ? (const VT*)h->rc_Ainv : nullptr;
-        if (nf) a.nf = *nf;
-    };
-    if (h->res_state == 1) {
-        ResidentArgs<VT> a;
-        fill(a);
-        *ran = launch_pcg_resident<VT>(h->res, a, h->stream) == 0;
-        if (!*ran) h->res_state = -1;
-    } else {
-        StreamArgs<VT> a;
-        fill(a);
-        a.ws = (VT*)h->str_ws; a.woff = h->str_woff; a.board = h->str_board;
-        *ran = launch_pcg_stream<VT>(h->str, a, h->stream) == 0;
-        if (!*ran) h->str_state = -1;
-    }
-    if (!*ran) cudaGetLastError();
     return SORS_OK;
 }
 
@@ -1523,7 +1533,7 @@ int pcg_one_launch_done(SorsHandle* h, bool refreshed, int* iters) {
         CK(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
         return fail(SORS_ERR_CUDA, "the PCG blocks did not meet within the limit");
     }
-    if (h->res_state == 1 ? h->res.coarse != 0 : true) {
+    if (h->res_ready ? h->res.coarse != 0 : true) {
         coarse_rate_check(h, refreshed, &h->rc_ref_rate, &h->rc_ready);
         coarse_state_check(h, refreshed, &h->rc_ready);
     }
@@ -3198,8 +3208,9 @@ int sors_create(const double* X, int32_t n_nodes, const int32_t* conn, int32_t n
 
 // Not part of the ABI: pick_parts for the tests, out = {form, G, A}.
 void sors_pcg_parts(int32_t n_nodes, int32_t n_elems, int32_t nodes_per_elem, int32_t value_bytes, int32_t sms,
-                    int32_t max_blocks, int32_t two_level, int32_t* out) {
-    const Parts p = pick_parts(n_nodes, n_elems, nodes_per_elem, (size_t)value_bytes, sms, max_blocks, two_level != 0);
+                    int32_t max_blocks, int32_t two_level, int32_t after, int32_t* out) {
+    const Parts p =
+        pick_parts(n_nodes, n_elems, nodes_per_elem, (size_t)value_bytes, sms, max_blocks, two_level != 0, after);
     out[0] = p.form; out[1] = p.G; out[2] = p.A;
 }
 

@@ -4,13 +4,13 @@ import ctypes as C
 import pytest
 
 
-def parts(n, e, nv=4, vsize=4, sms=148, cap=0, two_level=1):
+def parts(n, e, nv=4, vsize=4, sms=148, cap=0, two_level=1, after=0):
     from sors_b200 import _lib
     fn = _lib.load().sors_pcg_parts
     fn.restype = None
-    fn.argtypes = [C.c_int32] * 7 + [C.POINTER(C.c_int32)]
+    fn.argtypes = [C.c_int32] * 8 + [C.POINTER(C.c_int32)]
     out = (C.c_int32 * 3)()
-    fn(n, e, nv, vsize, sms, cap, two_level, out)
+    fn(n, e, nv, vsize, sms, cap, two_level, after, out)
     return tuple(out)
 
 
@@ -30,3 +30,19 @@ def test_grid_cap_holds_for_the_cluster(n, e, nv, vsize, cap):
 @pytest.mark.parametrize("cap", [1184, 14_510_025, 2**31 - 1])
 def test_cap_above_the_whole_gpu_changes_nothing(cap):
     assert parts(9856, 52488, cap=cap) == parts(9856, 52488)
+
+
+@pytest.mark.parametrize("n,e,nv,vsize,forms", [(525, 1536, 4, 8, [1, 2, 3]), (9856, 52488, 4, 4, [2, 3]),
+                                                (39304, 215622, 4, 8, [2, 3]), (101000, 576000, 4, 4, [3]),
+                                                (18921, 15680, 8, 8, [2])])
+def test_a_refused_form_goes_on_to_the_next(n, e, nv, vsize, forms):
+    """Forms in their order, each at most once, down to none (the rings of FP64 hex rows are too
+    large to stream); the streamed one needs the coarse correction."""
+    seen, form = [], 0
+    while True:
+        form = parts(n, e, nv, vsize, after=form)[0]
+        if not form:
+            break
+        seen.append(form)
+    assert seen == forms
+    assert 3 not in [parts(n, e, nv, vsize, two_level=0, after=k)[0] for k in range(4)]
