@@ -306,9 +306,12 @@ cudaError_t dzero(SorsHandle* h, void* dst, size_t bytes) {
     return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
 }
 
+// For the tests (sors_test_deny): how many device allocations of this thread fail next.
+thread_local int t_deny_allocs = 0;
+
 int dalloc(SorsHandle* h, void** p, size_t bytes) {
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMalloc(p, bytes);
+    cudaError_t e = t_deny_allocs > 0 && t_deny_allocs-- ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
         *p = nullptr;
         return fail(SORS_ERR_OOM, std::string("device allocation of ") + std::to_string(bytes) +
@@ -1451,12 +1454,14 @@ int plan_stream(SorsHandle* h) {
 
 // The plan of the handle's form, made at the first solve that could use it.  The form
 // was chosen by the mesh's size alone; one that its rows and borders refuse (a range of
-// many short rows, as of nodes without elements; borders of an unordered mesh) goes on
-// to the next, and past the last to the launches per kernel.
+// many short rows, as of nodes without elements; borders of an unordered mesh), or that
+// the device has no room for, goes on to the next, and past the last to the launches
+// per kernel.
 int plan_one_launch(SorsHandle* h) {
     while (h->parts_form && !h->res_ready && !h->str_ready) {
         const int st = h->parts_form == 3 ? plan_stream(h) : plan_resident(h);
-        if (st) return st;
+        if (st == SORS_ERR_OOM) cudaGetLastError();
+        else if (st) return st;
         h->rc_ready = false;
         if (!h->res_ready && !h->str_ready) choose_parts(h, h->parts_form);
     }
@@ -3213,6 +3218,9 @@ void sors_pcg_parts(int32_t n_nodes, int32_t n_elems, int32_t nodes_per_elem, in
         pick_parts(n_nodes, n_elems, nodes_per_elem, (size_t)value_bytes, sms, max_blocks, two_level != 0, after);
     out[0] = p.form; out[1] = p.G; out[2] = p.A;
 }
+
+// Not part of the ABI: the next `count` device allocations of this thread fail.
+void sors_test_deny(int32_t count) { t_deny_allocs = count; }
 
 void sors_destroy(SorsHandle* h) {
     if (!h) return;

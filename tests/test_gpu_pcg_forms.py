@@ -9,7 +9,7 @@ from sors_b200 import meshes
 pytestmark = pytest.mark.gpu
 
 
-def _step(X, T, E, solver):
+def _step(X, T, E, solver, deny=0):
     from sors_b200 import _lib
     from sors_b200 import py_sors as ps
     s = ps.SimulationSettings()
@@ -28,7 +28,11 @@ def _step(X, T, E, solver):
     en.set_initial_velocity(np.where(mask == 1, 0.0, v))
     sol = ps.Solver(s)
     n0 = _lib.load().sors_kernel_launch_count()
-    q = sol.step(X.ravel(), en)
+    _lib.load().sors_test_deny(deny)
+    try:
+        q = sol.step(X.ravel(), en)
+    finally:
+        _lib.load().sors_test_deny(0)
     return q, _lib.load().sors_kernel_launch_count() - n0, sol.last_stats
 
 
@@ -40,4 +44,14 @@ def test_range_with_too_many_rows():
     X, T = np.concatenate([far, X]), T + 600
     q, launches, st = _step(X, T, E, "pcg")
     assert launches < st.pcg_iters
+    assert np.abs(q - _step(X, T, E, "minres")[0]).max() <= 1e-8
+
+
+@pytest.mark.parametrize("cells,deny,one_launch", [((20, 21, 21), 1, True), ((20, 21, 21), 2, False),
+                                                   ((7, 8, 6), 1, True), ((7, 8, 6), 3, False)])
+def test_no_room_for_the_plan(cells, deny, one_launch):
+    """The plan's allocation fails on the device, once or for every form: the step is made all the same."""
+    X, T, E = meshes.jittered_block_tets(*cells, tuple(5e-3 * c for c in cells), jitter=0.1, seed=5)
+    q, launches, st = _step(X, T, E, "pcg", deny)
+    assert (launches < st.pcg_iters) == one_launch
     assert np.abs(q - _step(X, T, E, "minres")[0]).max() <= 1e-8
