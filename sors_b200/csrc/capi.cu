@@ -17,10 +17,12 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <new>
 #include <functional>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <limits>
 #include <vector>
@@ -306,8 +308,9 @@ cudaError_t dzero(SorsHandle* h, void* dst, size_t bytes) {
     return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
 }
 
-// For the tests (sors_test_deny): how many device allocations of this thread fail next.
-thread_local int t_deny_allocs = 0;
+// For the tests (sors_test_deny): how many device allocations and thread starts of this
+// thread fail next.
+thread_local int t_deny_allocs = 0, t_deny_threads = 0;
 
 int dalloc(SorsHandle* h, void** p, size_t bytes) {
     if (bytes == 0) bytes = 16;
@@ -367,6 +370,38 @@ void parallel_for(int n, F&& f) {
         ts.emplace_back([&f, a, b]() { f(a, b); });
     }
     for (auto& t : ts) t.join();
+}
+
+// A thread that runs f; false when the host starts no more.
+template <typename F>
+bool start_thread(std::thread& t, F&& f) {
+    if (t_deny_threads > 0 && t_deny_threads--) return false;
+    try {
+        t = std::thread(std::forward<F>(f));
+    } catch (const std::system_error&) {
+        return false;
+    }
+    return true;
+}
+
+// f(k) for k < n, on as many threads as the host starts.  An exception of any comes
+// out of here as std::bad_alloc, when all have ended.
+template <typename F>
+void on_threads(int n, F&& f) {
+    std::atomic<bool> failed{false};
+    auto run = [&](int k) {
+        try {
+            f(k);
+        } catch (const std::exception&) {
+            failed = true;
+        }
+    };
+    std::vector<std::thread> ts(std::max(0, n - 1));
+    int k = 0;
+    while (k < n - 1 && start_thread(ts[k], [&run, k]() { run(k); })) k++;
+    for (int j = k; j < n; j++) run(j);
+    for (int j = 0; j < k; j++) ts[j].join();
+    if (failed) throw std::bad_alloc();
 }
 
 // Host copies of the pattern's pair lists and slot items (set-up only).
@@ -1339,34 +1374,31 @@ int plan_stream(SorsHandle* h) {
     std::vector<std::vector<int>> halos(G);
     std::vector<std::vector<int2>> abs_(G);
     const int nt = (int)std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-    std::vector<std::thread> ts;
-    for (int k = 0; k < nt; k++)
-        ts.emplace_back([&, k]() {
-            std::vector<int> seen(N, -1), local(N), met(nagg, -1);
-            for (int b = k; b < G; b += nt) {
-                const int a0 = row0[b], a1 = row0[b + 1];
-                std::vector<int>& hl = halos[b];
-                for (int i = a0; i < a1; i++)
-                    for (int c = rp[i]; c < rp[i + 1]; c++) {
-                        const int j = h->col_h[c];
-                        if (met[aid[j]] != aid[i]) {
-                            met[aid[j]] = aid[i];
-                            abs_[b].push_back(make_int2(aid[i], aid[j]));
-                        }
-                        if (j >= a0 && j < a1) {
-                            lcol[c] = (uint16_t)(j - a0);
-                            continue;
-                        }
-                        if (seen[j] != b) {
-                            seen[j] = b;
-                            local[j] = (int)hl.size() + a1 - a0;
-                            hl.push_back(j);
-                        }
-                        lcol[c] = (uint16_t)local[j];
+    on_threads(nt, [&](int k) {
+        std::vector<int> seen(N, -1), local(N), met(nagg, -1);
+        for (int b = k; b < G; b += nt) {
+            const int a0 = row0[b], a1 = row0[b + 1];
+            std::vector<int>& hl = halos[b];
+            for (int i = a0; i < a1; i++)
+                for (int c = rp[i]; c < rp[i + 1]; c++) {
+                    const int j = h->col_h[c];
+                    if (met[aid[j]] != aid[i]) {
+                        met[aid[j]] = aid[i];
+                        abs_[b].push_back(make_int2(aid[i], aid[j]));
                     }
-            }
-        });
-    for (auto& t : ts) t.join();
+                    if (j >= a0 && j < a1) {
+                        lcol[c] = (uint16_t)(j - a0);
+                        continue;
+                    }
+                    if (seen[j] != b) {
+                        seen[j] = b;
+                        local[j] = (int)hl.size() + a1 - a0;
+                        hl.push_back(j);
+                    }
+                    lcol[c] = (uint16_t)local[j];
+                }
+        }
+    });
     std::vector<int> halo_ptr(G + 1, 0), halo;
     std::vector<uint8_t> border(N, 0);
     std::vector<int2> ab;
@@ -1455,11 +1487,16 @@ int plan_stream(SorsHandle* h) {
 // The plan of the handle's form, made at the first solve that could use it.  The form
 // was chosen by the mesh's size alone; one that its rows and borders refuse (a range of
 // many short rows, as of nodes without elements; borders of an unordered mesh), or that
-// the device has no room for, goes on to the next, and past the last to the launches
+// device or host have no room for, goes on to the next, and past the last to the launches
 // per kernel.
 int plan_one_launch(SorsHandle* h) {
     while (h->parts_form && !h->res_ready && !h->str_ready) {
-        const int st = h->parts_form == 3 ? plan_stream(h) : plan_resident(h);
+        int st;
+        try {
+            st = h->parts_form == 3 ? plan_stream(h) : plan_resident(h);
+        } catch (const std::exception&) {
+            st = SORS_ERR_OOM;  // of the host's memory: no exception leaves a C entry
+        }
         if (st == SORS_ERR_OOM) cudaGetLastError();
         else if (st) return st;
         h->rc_ready = false;
@@ -2965,9 +3002,11 @@ void number_by_parts(SorsHandle* h, const double* X, std::vector<int>& n2o) {
         const int half = (g1 - g0) / 2, m = a + (int)((int64_t)(b - a) * half / (g1 - g0));
         if (m > a && m < b) split(a, b, m);
         if (depth < 3 && b - a > 4000) {
-            std::thread t([&]() { ranges(a, m, g0, g0 + half, depth + 1); });
+            std::thread t;
+            const bool started = start_thread(t, [&]() { ranges(a, m, g0, g0 + half, depth + 1); });
             ranges(m, b, g0 + half, g1, depth + 1);
-            t.join();
+            if (started) t.join();
+            else ranges(a, m, g0, g0 + half, depth + 1);
         } else {
             ranges(a, m, g0, g0 + half, depth);
             ranges(m, b, g0 + half, g1, depth);
@@ -3219,8 +3258,11 @@ void sors_pcg_parts(int32_t n_nodes, int32_t n_elems, int32_t nodes_per_elem, in
     out[0] = p.form; out[1] = p.G; out[2] = p.A;
 }
 
-// Not part of the ABI: the next `count` device allocations of this thread fail.
-void sors_test_deny(int32_t count) { t_deny_allocs = count; }
+// Not part of the ABI: the calling thread's next device allocations and thread starts fail.
+void sors_test_deny(int32_t allocations, int32_t threads) {
+    t_deny_allocs = allocations;
+    t_deny_threads = threads;
+}
 
 void sors_destroy(SorsHandle* h) {
     if (!h) return;

@@ -9,7 +9,7 @@ from sors_b200 import meshes
 pytestmark = pytest.mark.gpu
 
 
-def _step(X, T, E, solver, deny=0):
+def _step(X, T, E, solver, deny=0, threads=0):
     from sors_b200 import _lib
     from sors_b200 import py_sors as ps
     s = ps.SimulationSettings()
@@ -28,11 +28,11 @@ def _step(X, T, E, solver, deny=0):
     en.set_initial_velocity(np.where(mask == 1, 0.0, v))
     sol = ps.Solver(s)
     n0 = _lib.load().sors_kernel_launch_count()
-    _lib.load().sors_test_deny(deny)
+    _lib.load().sors_test_deny(deny, threads)
     try:
         q = sol.step(X.ravel(), en)
     finally:
-        _lib.load().sors_test_deny(0)
+        _lib.load().sors_test_deny(0, 0)
     return q, _lib.load().sors_kernel_launch_count() - n0, sol.last_stats
 
 
@@ -55,3 +55,12 @@ def test_no_room_for_the_plan(cells, deny, one_launch):
     q, launches, st = _step(X, T, E, "pcg", deny)
     assert (launches < st.pcg_iters) == one_launch
     assert np.abs(q - _step(X, T, E, "minres")[0]).max() <= 1e-8
+
+
+@pytest.mark.parametrize("threads", [1, 100])
+def test_no_threads_for_the_plan(threads):
+    """The host starts some or none of the streamed plan's threads: the plan is made on those that there are."""
+    X, T, E = meshes.jittered_block_tets(20, 21, 21, (0.1, 0.105, 0.105), jitter=0.1, seed=5)
+    a, launches, st = _step(X, T, E, "pcg", 1, threads)
+    assert launches < st.pcg_iters
+    assert np.array_equal(a, _step(X, T, E, "pcg", 1)[0])
