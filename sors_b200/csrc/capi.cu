@@ -220,6 +220,7 @@ struct SorsHandle {
     bool res_ready = false, str_ready = false;
     ResidentPlan res;
     unsigned long long *res_zg = nullptr, *res_box = nullptr;
+    unsigned long long pcg_wait_ns = 1000000000ull;  // limit of each wait between its blocks
     unsigned* res_epoch = nullptr;
     // its two-level preconditioner: one aggregate per row range
     CoarseArgs rcargs;
@@ -1541,6 +1542,7 @@ int pcg_one_launch(SorsHandle* h, double eta, double abs_tol, const double* g, c
             a.x = (VT*)h->x; a.p0 = (VT*)h->p0; a.p1 = (VT*)h->p1; a.zg = h->res_zg; a.box = h->res_box;
             a.eta2 = eta * eta; a.abs_tol2 = abs_tol * abs_tol; a.maxit = h->s.pcg_max_iter;
             a.pflag = h->proj_flag; a.pn = h->proj_n; a.epoch = h->res_epoch; a.sc = h->sc;
+            a.wait_ns = h->pcg_wait_ns;
             a.fixed = h->node_mask;
             a.Ainv = coarse ? (const VT*)h->rc_Ainv : nullptr;
             if (nf) a.nf = *nf;
@@ -3263,6 +3265,10 @@ void sors_test_deny(int32_t allocations, int32_t threads) {
     t_deny_allocs = allocations;
     t_deny_threads = threads;
 }
+
+// Not part of the ABI: the limit of the waits of the handle's one-launch PCG (0: a
+// single look, so that a wait runs out).
+void sors_test_pcg_wait(SorsHandle* h, uint64_t ns) { h->pcg_wait_ns = ns; }
 
 void sors_destroy(SorsHandle* h) {
     if (!h) return;

@@ -16,8 +16,27 @@ constexpr int kWarps = kT / 32;
 constexpr int kBoxes = kResidentBoxEntries;  // mailbox entries: five per polling lane
 constexpr int kScratch = 3328;
 constexpr int kPollLimit = 1 << 21;          // about a second
-static_assert(kResidentMaxBlocks <= kBoxes && kBoxes % 32 == 0, "a lane polls kBoxes / 32 entries");
 typedef unsigned long long u64;
+
+// The limit of a wait, in elapsed time: one look at the clock in 256 at the value
+// waited for, the first of which starts it.  Limit 0: a single look at the value.
+struct Patience {
+    u64 t0 = 0;
+    unsigned n;
+    __device__ __forceinline__ explicit Patience(u64 limit_ns) : n(limit_ns ? 0u : 255u) {}
+    __device__ __forceinline__ bool clock(u64 limit_ns) {
+        u64 t;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        if (n == 256u) t0 = t;
+        return t - t0 < limit_ns;
+    }
+    __device__ __forceinline__ bool more(u64 limit_ns) { return (++n & 255u) || clock(limit_ns); }
+    // the same answer in every lane of the warp
+    __device__ __forceinline__ bool more_warp(u64 limit_ns) {
+        return (++n & 255u) || __shfl_sync(0xffffffffu, (int)clock(limit_ns), 0);
+    }
+};
+static_assert(kResidentMaxBlocks <= kBoxes && kBoxes % 32 == 0, "a lane polls kBoxes / 32 entries");
 
 // values per node of a column's p: one 16-byte load (FP32), three 8-byte loads (FP64)
 template <typename VT>
@@ -81,7 +100,10 @@ struct Scratch {
     double tot[2];
     double irz;                    // 1 / r.z
     double zc[6][2];               // the range's coarse correction, two partial sums each
-    int abort, pad;
+    // A wait ran out.  abort is set between the two barriers of an exchange and read
+    // after the second, so the block's threads agree; late by the waits between
+    // exchanges, and becomes abort in the next one.
+    int abort, late;
     double slot[kVals][16];  // cluster form: the blocks' messages, by value
 };
 static_assert(sizeof(Scratch) <= kScratch, "fixed scratch");
@@ -94,10 +116,10 @@ static_assert(sizeof(Scratch) <= kScratch, "fixed scratch");
 // in a row, so a slot or mailbox entry is written again only after every block
 // has read it.
 // halo_bytes: border z the block receives with site 1 (cluster form).  False:
-// something did not arrive within the poll limit.
+// something did not arrive within the limit (every thread of the block alike).
 template <int SITE, int NV, int NSUM, bool CL>
 __device__ __forceinline__ bool exchange(double (&v)[NSUM ? NSUM : 1], Scratch* sh, int G, unsigned epoch, u64* box,
-                                         unsigned parity, int halo_bytes, double* yq) {
+                                         unsigned parity, int halo_bytes, double* yq, u64 limit_ns) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, me = blockIdx.x;
     __syncthreads();
     if (w < NV) {
@@ -126,7 +148,7 @@ __device__ __forceinline__ bool exchange(double (&v)[NSUM ? NSUM : 1], Scratch* 
             const u64* q = box + (((size_t)me * kVals + at) * G + l) * 2;
             u64 a[J], b[J];
             bool ok;
-            int n = 0;
+            Patience wait(limit_ns);
             do {
                 ok = true;
 #pragma unroll
@@ -136,7 +158,7 @@ __device__ __forceinline__ bool exchange(double (&v)[NSUM ? NSUM : 1], Scratch* 
                 for (int j = 0; j < J; j++)
                     if (l + 32 * j < G) ok = ok && has(a[j], epoch) && has(b[j], epoch);
                 ok = __all_sync(0xffffffffu, ok);  // the warp stays together
-            } while (!ok && ++n < kPollLimit);
+            } while (!ok && wait.more_warp(limit_ns));
             if (w < NSUM) {
                 double t = 0.0;
 #pragma unroll
@@ -153,6 +175,7 @@ __device__ __forceinline__ bool exchange(double (&v)[NSUM ? NSUM : 1], Scratch* 
             if (l == 0 && !ok) sh->abort = 1;
         }
     }
+    if (!CL && threadIdx.x == kT - 1 && sh->late) sh->abort = 1;
     if constexpr (CL) {
         const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh->bar[SITE]);
         unsigned got = 0;

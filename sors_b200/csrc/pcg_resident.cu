@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
     const int h0 = pl.halo_ptr[me], nh = pl.halo_ptr[me + 1] - h0;
     unsigned epoch = CL ? 0u : *(volatile const unsigned*)a.epoch;
     if (t == 0) {
-        sh->abort = 0;
+        sh->abort = sh->late = 0;
         if constexpr (CL)
 #pragma unroll
             for (int k = 0; k < 3; k++)
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
             for (int s = 16; s > 0; s >>= 1) c[m] += __shfl_xor_sync(0xffffffffu, c[m], s);
             if (lane == 0) sh->part[t >> 5][m] = c[m];
         }
-        const bool here = exchange<2, 6, 0, CL>(none, sh, G, ++epoch, a.box, par2, 0, syc + 2 * nc);
+        const bool here = exchange<2, 6, 0, CL>(none, sh, G, ++epoch, a.box, par2, 0, syc + 2 * nc, a.wait_ns);
         par2 ^= 1u;
         coarse(true, 0.0, nullptr, syc + cur * nc);
         return here;
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
     double d1[1] = {0.0}, acc[2];
     if constexpr (TL) ok = renew();
     precondition();
-    ok = exchange<1, 2, 2, CL>(acc, sh, G, ++epoch, a.box, par1, nh * kZBytes, nullptr) && ok;
+    ok = exchange<1, 2, 2, CL>(acc, sh, G, ++epoch, a.box, par1, nh * kZBytes, nullptr, a.wait_ns) && ok;
     par1 ^= 1u;
     double rz = acc[0], rr = acc[1], pq = 0.0, alpha = 0.0, beta = 0.0;
     const double bnorm2 = rr;
@@ -363,15 +363,15 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
                 const u64* q = a.zg + Z * (size_t)shalo[k];
                 u64 w[Z];
                 bool here;
-                int n = 0;
+                Patience wait(a.wait_ns);
                 do {
                     here = true;
 #pragma unroll
                     for (int m = 0; m < Z; m += 2) ld_words(q + m, w[m], w[m + 1]);
 #pragma unroll
                     for (int m = 0; m < Z; m++) here = here && has(w[m], epoch);
-                } while (!here && ++n < kPollLimit);
-                if (!here) sh->abort = 1;
+                } while (!here && wait.more(a.wait_ns));
+                if (!here) sh->late = 1;
                 if constexpr (sizeof(VT) == 4) {
 #pragma unroll
                     for (int m = 0; m < 3; m++) zz[m] = (VT)__uint_as_float((unsigned)w[m]);
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
 #pragma unroll
                 for (int m = 0; m < 6; m++) sh->part[t >> 5][1 + m] = yw[m];
         }
-        ok = exchange<0, TL ? kMsg : 1, 1, CL>(d1, sh, G, ++epoch, a.box, par0, 0, syc + 2 * nc);
+        ok = exchange<0, TL ? kMsg : 1, 1, CL>(d1, sh, G, ++epoch, a.box, par0, 0, syc + 2 * nc, a.wait_ns);
         par0 ^= 1u;
         if (!ok) break;
         pq = d1[0];
@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
             }
         }
         precondition();
-        ok = exchange<1, 2, 2, CL>(acc, sh, G, ++epoch, a.box, par1, nh * kZBytes, nullptr);
+        ok = exchange<1, 2, 2, CL>(acc, sh, G, ++epoch, a.box, par1, nh * kZBytes, nullptr, a.wait_ns);
         par1 ^= 1u;
         if (!ok) break;
         beta = acc[0] * sh->irz;
@@ -506,12 +506,13 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
     // no block leaves while another may still push into its shared memory
     if constexpr (CL) cg::this_cluster().sync();
     else __syncthreads();
+    // a wait of any block that ran out fails the solve
+    if (t == 0 && (sh->abort | sh->late)) atomicOr(&a.sc->status, kFlagTimeout);
     if (me == 0 && t == 0) {
         DevScalars* sc = a.sc;
         sc->rz = rz; sc->rr = rr; sc->bnorm2 = bnorm2; sc->tol2 = tol2; sc->pq = pq;
         sc->alpha = breakdown ? 0.0 : alpha; sc->beta = beta;
         sc->it = it; sc->maxit = a.maxit; sc->breakdown = breakdown; sc->done = 1; sc->skip = 0;
-        if (sh->abort) sc->status |= kFlagTimeout;
         if (!CL) *a.epoch = epoch;
     }
 }

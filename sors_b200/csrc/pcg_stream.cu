@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
     unsigned epoch = *(volatile const unsigned*)a.epoch;
     unsigned char* ring = smem + o.ring + (size_t)w * pl.depth * pl.group_bytes;
     const unsigned bars = sptr(smem + o.bar) + 8u * (unsigned)(w * pl.depth);
-    if (t == 0) sh->abort = 0;
+    if (t == 0) sh->abort = sh->late = 0;
     if (lane == 0)
         for (int k = 0; k < pl.depth; k++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8u * k) : "memory");
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
     double acc[2], d1[1];
     update(VT(0), VT(0), true);
     prefetch();
-    ok = exchange<1, 2, 2, false>(acc, sh, G, ++epoch, a.box, 0u, 0, nullptr) && ok;
+    ok = exchange<1, 2, 2, false>(acc, sh, G, ++epoch, a.box, 0u, 0, nullptr, a.wait_ns) && ok;
     double rz = acc[0], rr = acc[1], pq = 0.0, alpha = 0.0, beta = 0.0;
     const double bnorm2 = rr;
     const double te = eta2 * rr, tol2 = te > abs_tol2 ? te : abs_tol2;
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
         u64* board = a.board + (flip ? board_words : 0);
         flip ^= 1;
         post(board, epoch);
-        ok = exchange<0, 1, 1, false>(d1, sh, G, epoch, a.box, 0u, 0, nullptr);
+        ok = exchange<0, 1, 1, false>(d1, sh, G, epoch, a.box, 0u, 0, nullptr, a.wait_ns);
         if (!ok) break;
         pq = d1[0];
         if (!(pq > 0.0)) {
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
             update(al, al, true);
         }
         prefetch();
-        ok = exchange<1, 2, 2, false>(acc, sh, G, ++epoch, a.box, 0u, 0, nullptr);
+        ok = exchange<1, 2, 2, false>(acc, sh, G, ++epoch, a.box, 0u, 0, nullptr, a.wait_ns);
         if (!ok) break;
         beta = acc[0] / rz;
         rz = acc[0];

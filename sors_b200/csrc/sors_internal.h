@@ -238,6 +238,7 @@ struct ResidentArgs {
     unsigned long long* zg = nullptr;   // grid form: published z, 4 (FP32) or 6 (FP64) words per node
     unsigned long long* box = nullptr;  // grid form: mailboxes, G kResidentBoxWords per block
     unsigned* epoch = nullptr;          // grid form: the last epoch used
+    unsigned long long wait_ns = 0;     // limit of each wait
     DevScalars* sc = nullptr;
 };
 // A whole two-level PCG solve in one launch with the matrix streaming through
@@ -280,6 +281,7 @@ struct StreamArgs {
     unsigned long long *zg = nullptr, *box = nullptr;
     unsigned long long* board = nullptr;  // three boards of nc entries, two words each
     unsigned* epoch = nullptr;
+    unsigned long long wait_ns = 0;
     DevScalars* sc = nullptr;
 };
 size_t stream_smem(const StreamPlan& pl, int vsize);
