@@ -18,6 +18,12 @@ constexpr int kScratch = 3328;
 constexpr int kPollLimit = 1 << 21;          // about a second
 typedef unsigned long long u64;
 
+__device__ __forceinline__ u64 clock_ns() {
+    u64 t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
 // The limit of a wait, in elapsed time: one look at the clock in 256 at the value
 // waited for, the first of which starts it.  Limit 0: a single look at the value.
 struct Patience {
@@ -25,8 +31,7 @@ struct Patience {
     unsigned n;
     __device__ __forceinline__ explicit Patience(u64 limit_ns) : n(limit_ns ? 0u : 255u) {}
     __device__ __forceinline__ bool clock(u64 limit_ns) {
-        u64 t;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        const u64 t = clock_ns();
         if (n == 256u) t0 = t;
         return t - t0 < limit_ns;
     }

@@ -40,6 +40,7 @@ namespace {
 
 constexpr int kMaxA = kStreamMaxAgg, kLPR = kStreamLanes;
 constexpr int kGR = 32 / kLPR;  // rows per group
+constexpr u64 kDrainNs = 1000000000ull;  // limit of the wait for a block's own copies
 
 struct SOff {
     int zc, part, y, a, sp, srp, halo, bar, ring;
@@ -63,16 +64,22 @@ __host__ __device__ inline SOff soffsets(const StreamPlan& pl) {
 
 __device__ __forceinline__ unsigned sptr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
-// Waits for phase `parity` of the barrier; false after the limit.
-__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
-    unsigned got = 0;
-    for (int n = 0; n < kPollLimit && !got; n++)
+// Waits for phase `parity` of the barrier; false after the limit (a try_wait that
+// fails has waited for some time itself).
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, u64 limit_ns) {
+    u64 t0 = 0;
+    for (;;) {
+        unsigned got;
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
             : "=r"(got)
             : "r"(bar), "r"(parity)
             : "memory");
-    return got != 0;
+        if (got) return true;
+        const u64 t = clock_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 >= limit_ns) return false;
+    }
 }
 
 __device__ __forceinline__ void bulk(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
@@ -113,7 +120,8 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8u * k) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    unsigned ring_phase = 0;  // bit k: the phase that slot k's next wait expects
+    // bit k: the phase that slot k's next wait expects; a copy into it has not been waited for
+    unsigned ring_phase = 0, ring_busy = 0;
     unsigned long long policy = 0;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     for (int i = t; i <= nr; i += kT) srp[i] = a.row_ptr[r0 + i] - b0;
@@ -194,13 +202,13 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
     auto coarse = [&](const u64* board, unsigned tag, bool fresh, double al) {
         for (int j = t; j < nc; j += kT) {
             u64 lo, hi;
-            int n = 0;
+            Patience wait(a.wait_ns);
             bool here;
             do {
                 ld_words(board + 2 * (size_t)j, lo, hi);
                 here = has(lo, tag) && has(hi, tag);
-            } while (!here && ++n < kPollLimit);
-            if (!here) sh->abort = 1;
+            } while (!here && wait.more(a.wait_ns));
+            if (!here) sh->late = 1;
             const double v = join(lo, hi);
             y[j] = fresh ? v : y[j] - al * v;
         }
@@ -251,7 +259,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
         ++epoch;
         post(a.board + 2 * board_words, epoch);
         coarse(a.board + 2 * board_words, epoch, true, 0.0);
-        return sh->abort == 0;
+        return sh->late == 0;  // set again only beyond the next exchange
     };
     // x += ax p, r -= ar q, z = M^-1 r + P zc published with the coming site-1 sum; r.z, r.r
     auto update = [&](VT ax, VT ar, bool with_z) {
@@ -336,8 +344,8 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
     };
     const int ngrp = (nr + kGR - 1) / kGR;
     const int sub = lane / kLPR, sl = lane % kLPR;
-    // fetches group gi into slot k of the warp's ring (one lane): matrix blocks,
-    // column indices, rows' offsets
+    // fetches group gi into slot k of the warp's ring: matrix blocks, column indices,
+    // rows' offsets
     auto fetch = [&](int gi, int k) {
         const int i0 = gi * kGR, i1 = min(i0 + kGR, nr);
         const size_t n0 = (size_t)b0 + srp[i0], n1 = (size_t)b0 + srp[i1];
@@ -359,12 +367,12 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
         bulk(dst + pl.slot_off, reinterpret_cast<const char*>(a.woff + r0 + i0), ob, bar);
     };
     // fills the ring for the next product (the matrix does not change: ahead of p)
-    bool filled = false;
     auto prefetch = [&]() {
-        filled = true;
-        if (lane == 0)
-            for (int k = 0; k < pl.depth; k++)
-                if (w + k * kWarps < ngrp) fetch(w + k * kWarps, k);
+        for (int k = 0; k < pl.depth; k++)
+            if (w + k * kWarps < ngrp) {
+                ring_busy |= 1u << k;
+                if (lane == 0) fetch(w + k * kWarps, k);
+            }
     };
     bool ok = renew();
     double acc[2], d1[1];
@@ -390,7 +398,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
         for (int kb = t; kb < nh; kb += HU * kT) {
             u64 wd[HU][Z];
             bool here;
-            int n = 0;
+            Patience wait(a.wait_ns);
             do {
                 here = true;
 #pragma unroll
@@ -405,8 +413,8 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
                     if (kb + u * kT < nh)
 #pragma unroll
                         for (int m = 0; m < Z; m++) here = here && has(wd[u][m], epoch);
-            } while (!here && ++n < kPollLimit);
-            if (!here) sh->abort = 1;
+            } while (!here && wait.more(a.wait_ns));
+            if (!here) sh->late = 1;
 #pragma unroll
             for (int u = 0; u < HU; u++)
                 if (kb + u * kT < nh) {
@@ -431,8 +439,15 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
             const int i = gi * kGR + sub, an = gi * kGR / L;
             if (an != ag) { flush(ag, yw, kLPR); ag = an; }
             const int ii = min(i, nr - 1), k0 = srp[ii], k1 = i < nr ? srp[ii + 1] : k0, kg = srp[gi * kGR];
-            if (!bar_wait(bars + 8u * slot, (ring_phase >> slot) & 1u)) sh->abort = 1;
+            // without its copy the group has no indices: the product ends here, and the
+            // solve in the exchange behind it
+            if (!__all_sync(0xffffffffu, bar_wait(bars + 8u * slot, (ring_phase >> slot) & 1u, a.wait_ns))) {
+                sh->late = 1;
+                break;
+            }
             ring_phase ^= 1u << slot;
+            const bool next = gi + pl.depth * kWarps < ngrp;
+            if (!next) ring_busy &= ~(1u << slot);
             const unsigned char* rs_ = ring + (size_t)slot * pl.group_bytes;
             const VT* hg = reinterpret_cast<const VT*>(rs_ + (((size_t)b0 + kg) * BB & 15));
             const uint16_t* cg_ = reinterpret_cast<const uint16_t*>(rs_ + pl.slot_col + (((size_t)b0 + kg) * 2 & 15));
@@ -447,7 +462,7 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
                 a2 += h[6] * p0 + h[7] * p1 + h[8] * p2;
             }
             __syncwarp();
-            if (lane == 0 && gi + pl.depth * kWarps < ngrp) fetch(gi + pl.depth * kWarps, slot);
+            if (lane == 0 && next) fetch(gi + pl.depth * kWarps, slot);
             slot = slot + 1 == pl.depth ? 0 : slot + 1;
 #pragma unroll
             for (int s = kLPR / 2; s > 0; s >>= 1) {
@@ -470,7 +485,6 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
             }
         }
         __syncwarp();
-        filled = false;
         flush(ag, yw, kLPR);
 #pragma unroll
         for (int s = 16; s >= kLPR; s >>= 1) pqw += __shfl_xor_sync(0xffffffffu, pqw, s);
@@ -508,9 +522,8 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
         done = rr <= tol2 || it >= a.maxit || !(rr == rr);
     }
     // the bulk copies still in flight must land before the block leaves
-    if (filled)
-        for (int k = 0; k < pl.depth; k++)
-            if (w + k * kWarps < ngrp) bar_wait(bars + 8u * k, (ring_phase >> k) & 1u);
+    for (int k = 0; k < pl.depth; k++)
+        if ((ring_busy >> k) & 1u) bar_wait(bars + 8u * k, (ring_phase >> k) & 1u, kDrainNs);
     for (int i = t; i < nr; i += kT) {
         const long long row = r0 + i;
 #pragma unroll
@@ -522,12 +535,12 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_stream(StreamPlan pl, StreamArgs<
         }
     }
     __syncthreads();
+    if (t == 0 && (sh->abort | sh->late)) atomicOr(&a.sc->status, kFlagTimeout);
     if (me == 0 && t == 0) {
         DevScalars* sc = a.sc;
         sc->rz = rz; sc->rr = rr; sc->bnorm2 = bnorm2; sc->tol2 = tol2; sc->pq = pq;
         sc->alpha = breakdown ? 0.0 : alpha; sc->beta = beta;
         sc->it = it; sc->maxit = a.maxit; sc->breakdown = breakdown; sc->done = 1; sc->skip = 0;
-        if (sh->abort) sc->status |= kFlagTimeout;
         *a.epoch = epoch;
     }
 }

@@ -49,3 +49,9 @@ def _run(cells, precision, two_level):
 @pytest.mark.parametrize("two_level", ["auto", False])
 def test_grid(cells, precision, two_level):
     _run(cells, precision, two_level)
+
+
+# 49k and 107k nodes: one and two aggregates per range
+@pytest.mark.parametrize("cells,precision", [((40, 34, 33), "fp64"), ((57, 43, 41), "mixed")])
+def test_streamed(cells, precision):
+    _run(cells, precision, "auto")
