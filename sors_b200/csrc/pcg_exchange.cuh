@@ -15,7 +15,6 @@ constexpr int kT = kResidentThreads;
 constexpr int kWarps = kT / 32;
 constexpr int kBoxes = kResidentBoxEntries;  // mailbox entries: five per polling lane
 constexpr int kScratch = 3328;
-constexpr int kPollLimit = 1 << 21;          // about a second
 typedef unsigned long long u64;
 
 __device__ __forceinline__ u64 clock_ns() {
@@ -91,6 +90,34 @@ __device__ __forceinline__ void push(unsigned dst, unsigned bar, float a, float 
                  : "memory");
 }
 
+// Waits for phase `parity` of the block's own mbarrier; false after the limit (a
+// try_wait that fails has waited for some time itself).
+__device__ __forceinline__ bool cluster_wait(unsigned bar, unsigned parity, u64 limit_ns) {
+    unsigned got;
+    if (limit_ns == 0) {
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+            " selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(got)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        return got != 0;
+    }
+    u64 t0 = 0;
+    for (;;) {
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+            " selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(got)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (got) return true;
+        const u64 t = clock_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 >= limit_ns) return false;
+    }
+}
+
 // Exchange sites and their values: 0 p.q (and P^T q, six values, with the coarse
 // correction), 1 r.z and r.r, 2 P^T r (six values, coarse correction).
 constexpr int kMsg = 7;
@@ -105,8 +132,8 @@ struct Scratch {
     double tot[2];
     double irz;                    // 1 / r.z
     double zc[6][2];               // the range's coarse correction, two partial sums each
-    // A wait ran out.  abort is set between the two barriers of an exchange and read
-    // after the second, so the block's threads agree; late by the waits between
+    // A wait ran out.  Grid form: abort is set between the two barriers of an exchange
+    // and read after the second, so the block's threads agree; late by the waits between
     // exchanges, and becomes abort in the next one.
     int abort, late;
     double slot[kVals][16];  // cluster form: the blocks' messages, by value
@@ -121,7 +148,8 @@ static_assert(sizeof(Scratch) <= kScratch, "fixed scratch");
 // in a row, so a slot or mailbox entry is written again only after every block
 // has read it.
 // halo_bytes: border z the block receives with site 1 (cluster form).  False:
-// something did not arrive within the limit (every thread of the block alike).
+// something did not arrive within the limit; grid form: in every thread of the block
+// alike, cluster form: in the threads that waited in vain.
 template <int SITE, int NV, int NSUM, bool CL>
 __device__ __forceinline__ bool exchange(double (&v)[NSUM ? NSUM : 1], Scratch* sh, int G, unsigned epoch, u64* box,
                                          unsigned parity, int halo_bytes, double* yq, u64 limit_ns) {
@@ -182,15 +210,7 @@ __device__ __forceinline__ bool exchange(double (&v)[NSUM ? NSUM : 1], Scratch* 
     }
     if (!CL && threadIdx.x == kT - 1 && sh->late) sh->abort = 1;
     if constexpr (CL) {
-        const unsigned bar = (unsigned)__cvta_generic_to_shared(&sh->bar[SITE]);
-        unsigned got = 0;
-        for (int n = 0; n < kPollLimit && !got; n++)
-            asm volatile(
-                "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-                " selp.u32 %0, 1, 0, p;\n}"
-                : "=r"(got)
-                : "r"(bar), "r"(parity)
-                : "memory");
+        const bool got = cluster_wait((unsigned)__cvta_generic_to_shared(&sh->bar[SITE]), parity, limit_ns);
         if (!got) sh->abort = 1;
         // 16 values: a lane each (twice per warp), four shuffles
 #pragma unroll
@@ -199,7 +219,7 @@ __device__ __forceinline__ bool exchange(double (&v)[NSUM ? NSUM : 1], Scratch* 
         for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
             for (int s = 0; s < NSUM; s++) v[s] += __shfl_xor_sync(0xffffffffu, v[s], o);
-        return true;
+        return got;
     } else {
         __syncthreads();
 #pragma unroll

@@ -59,6 +59,8 @@ namespace sors {
 
 namespace {
 
+constexpr u64 kStayNs = 20000;  // a push takes about a microsecond
+
 // Byte offsets of a block's shared memory, the same in every block of a launch.
 struct Off {
     int sp, sq, sm, sx, sz, soff, sa, syc, sov, sgb, shalo, spp, spush, scol, sval;
@@ -343,18 +345,21 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
     const double te = eta2 * rr, tol2 = te > abs_tol2 ? te : abs_tol2;
     int it = 0, breakdown = 0;
     bool done = !ok || rr <= tol2 || a.maxit <= 0;
+    // Cluster form: no barrier lies between the sums and the threads that use them, and
+    // where a wait ran out they may differ, so what ends the solve is agreed on at one
+    // place, the barrier behind the border columns.
     // threads without a row take the border columns first
     const int nru = (nr + 31) & ~31;
     const int th = t >= nru ? t - nru : t + kT - nru;
-    while (!done) {
+    while (CL || !done) {
         // p at the range's own and border columns
         const VT bt = (VT)beta;
-        if (t < nr) {
+        if (t < nr && !(CL && done)) {
             VT* pc = sp + P * t;
 #pragma unroll
             for (int k = 0; k < 3; k++) pc[k] = zs[k] + bt * pc[k];
         }
-        for (int k = th; k < nh; k += kT) {
+        for (int k = CL && done ? nh : th; k < nh; k += kT) {
             VT zz[3];
             if constexpr (CL) {
 #pragma unroll
@@ -387,7 +392,11 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
         // a block barrier does not bring lanes together that left the loop apart,
         // and a warp in pieces runs what follows once per piece
         __syncwarp();
-        __syncthreads();
+        if constexpr (CL) {
+            if (__syncthreads_or(done)) break;
+        } else {
+            __syncthreads();
+        }
         // the coming beta's divisor, on a warp that has time: every thread has read the
         // last one before this barrier and reads this one after the sums' barriers
         if (t == kT - 1) sh->irz = 1.0 / rz;
@@ -456,15 +465,13 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
         }
         ok = exchange<0, TL ? kMsg : 1, 1, CL>(d1, sh, G, ++epoch, a.box, par0, 0, syc + 2 * nc, a.wait_ns);
         par0 ^= 1u;
-        if (!ok) break;
+        if (!CL && !ok) break;
         pq = d1[0];
-        if (!(pq > 0.0)) {
-            breakdown = 1;
-            break;
-        }
+        breakdown = !(pq > 0.0);
+        if (!CL && breakdown) break;
         alpha = rz / pq;
         const VT al = (VT)alpha;
-        if (t < nr) {
+        if (t < nr && !(CL && breakdown)) {
             VT q[3];
 #pragma unroll
             for (int k = 0; k < 3; k++) {
@@ -477,21 +484,27 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
         }
         if constexpr (TL) {
             if (sizeof(VT) == 4 && (it & 7) == 7) {
-                if (!renew()) break;
+                ok = renew() && ok;
+                if (!CL && !ok) break;
             } else {
                 coarse(false, (double)al, syc + cur * nc, syc + (cur ^ 1) * nc);
                 cur ^= 1;
             }
         }
         precondition();
-        ok = exchange<1, 2, 2, CL>(acc, sh, G, ++epoch, a.box, par1, nh * kZBytes, nullptr, a.wait_ns);
+        ok = exchange<1, 2, 2, CL>(acc, sh, G, ++epoch, a.box, par1, nh * kZBytes, nullptr, a.wait_ns) && ok;
         par1 ^= 1u;
-        if (!ok) break;
+        if (!CL && !ok) break;
         beta = acc[0] * sh->irz;
-        rz = acc[0];
         rr = acc[1];
         it++;
         done = rr <= tol2 || it >= a.maxit || !(rr == rr);
+        if (CL && (breakdown || !ok)) {
+            it -= breakdown;
+            done = true;
+        } else {
+            rz = acc[0];
+        }
     }
     if (t < nr) {
 #pragma unroll
@@ -503,9 +516,16 @@ __global__ void __launch_bounds__(kT, 1) k_pcg_resident(ResidentPlan pl, Residen
             for (int k = 0; k < 3; k++) pb[k] = sp[P * t + k];
         }
     }
-    // no block leaves while another may still push into its shared memory
-    if constexpr (CL) cg::this_cluster().sync();
-    else __syncthreads();
+    // no block leaves while another may still push into its shared memory: a solve that
+    // ends by its sums has received all that was sent to it, one that a wait ended stays
+    // for what may be on its way
+    if constexpr (CL) {
+        cg::this_cluster().sync();
+        if (t == 0 && sh->abort)
+            for (const u64 t0 = clock_ns(); clock_ns() - t0 < kStayNs;) {}
+    } else {
+        __syncthreads();
+    }
     // a wait of any block that ran out fails the solve
     if (t == 0 && (sh->abort | sh->late)) atomicOr(&a.sc->status, kFlagTimeout);
     if (me == 0 && t == 0) {

@@ -44,6 +44,13 @@ def _run(cells, precision, two_level):
     assert np.array_equal(sol.step(q, en), ref[0]) and sol.last_stats.pcg_iters == ref[1]
 
 
+# N = 81, 525 and 1,014: three blocks (no coarse correction) and sixteen
+@pytest.mark.parametrize("cells,precision", [((8, 2, 2), "mixed"), ((20, 4, 4), "fp64"), ((25, 12, 2), "mixed")])
+@pytest.mark.parametrize("two_level", ["auto", False])
+def test_cluster(cells, precision, two_level):
+    _run(cells, precision, two_level)
+
+
 # N = 4,225 and 9,856: eight and four lanes per row
 @pytest.mark.parametrize("cells,precision", [((24, 12, 12), "fp64"), ((27, 15, 21), "mixed")])
 @pytest.mark.parametrize("two_level", ["auto", False])
