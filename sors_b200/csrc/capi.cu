@@ -1146,6 +1146,9 @@ Parts pick_parts(int N, int E, int nv, size_t hs, int sms, int max_blocks, bool 
     // shared memory, and up to 2,500 rows a range (ms per step, launch per kernel /
     // streamed: 77,841 FP32 nodes 11.2 / 6.7, 169,781 17.5 / 12.9, FP64 24.1 / 16.5,
     // 291,870 25.3 / 19.8, 522,801 36.7 / 37.1).
+    // at least 32 rows a range, as an aggregate has: of fewer, the rigid-body modes are not
+    // independent, and what FP32 rounding makes of their matrix is no preconditioner
+    gmax = std::max(1, std::min(gmax, (N + 31) / 32));
     const double rows = (double)N / gmax, border = 7.0 * pow(rows, 2.0 / 3.0);
     const double ring = 16.0 * 8.0 * (nv == 4 ? 16.0 : 27.0) * (9.0 * hs + 2.0);
     if (rows > 2500.0 ||

@@ -46,3 +46,10 @@ def test_a_refused_form_goes_on_to_the_next(n, e, nv, vsize, forms):
         seen.append(form)
     assert seen == forms
     assert 3 not in [parts(n, e, nv, vsize, two_level=0, after=k)[0] for k in range(4)]
+
+
+@pytest.mark.parametrize("n", [8, 81, 525, 2000, 9856])
+@pytest.mark.parametrize("after", [0, 1, 2])
+def test_ranges_have_enough_rows_for_their_rigid_modes(n, after):
+    form, g, a = parts(n, 5 * n, after=after)
+    assert form and n > 16 * (g * a - 1)
