@@ -236,6 +236,7 @@ struct SorsHandle {
     void* rc_Ainv = nullptr;
     bool rc_ready = false;
     double rc_ref_rate = 0.0;
+    bool coarse_retry = false;          // the coarse operator was left out: build it for the next Hessian
     int tl_req = 0;  // settings.two_level as given (2: where it pays)
 
     double prev_gnorm = -1.0;
@@ -762,6 +763,7 @@ int eval_system(SorsHandle* h, double dt, bool want_hess, AsmMode mode = kAsmSte
     int st = compute_external(h);
     if (st) return st;
     (want_hess ? h->n_hess_evals : h->n_grad_evals)++;
+    if (want_hess && h->coarse_retry) h->rc_ready = h->tl_ready = h->coarse_retry = false;
     const int project = h->force_project >= 0 ? h->force_project
                         : (h->s.project_spd == 2 ? (h->proj_fallback ? 1 : 0) : h->s.project_spd);
     AsmArgs<HT> a = asm_args<HT>(h, dt, want_hess, mode, project);
@@ -1028,6 +1030,14 @@ int ensure_two_level(SorsHandle* h) {
     return setup_two_level(h, X.data());
 }
 
+// Inverts a coarse matrix in place; sc->coarse_bad says that it was indefinite (beyond
+// what rounding of the Hessian's values makes of a singular one).
+int invert_coarse(SorsHandle* h, int nc, double* Ac, const double* diag, double* work) {
+    CK(cudaMemsetAsync(&h->sc->coarse_bad, 0, sizeof(int), h->stream));
+    launch_coarse_invert(nc, Ac, diag, work, mixed(h) ? 1e-5 : 1e-10, &h->sc->coarse_bad, h->stream);
+    return SORS_OK;
+}
+
 // The coarse operator P^T H P of the Hessian in h->H, inverted in place.
 template <typename HT, typename VT>
 int build_coarse(SorsHandle* h) {
@@ -1039,8 +1049,9 @@ int build_coarse(SorsHandle* h) {
     else
         launch_coarse_galerkin_d(h->tl_npairs, h->tl_pair_ptr, h->tl_items, h->tl_ab, h->col, (const double*)h->H,
                                  h->nnzb, h->cargs, h->tl_Ac, h->tl_diag, h->stream);
-    launch_coarse_invert(nc, h->tl_Ac, h->tl_diag, h->tl_work, h->stream);
-    launch_to_vt_pad<VT>(nc, h->tl_ld, h->tl_Ac, (VT*)h->tl_Ainv, h->stream);
+    int st = invert_coarse(h, nc, h->tl_Ac, h->tl_diag, h->tl_work);
+    if (st) return st;
+    launch_to_vt_pad<VT>(nc, h->tl_ld, h->tl_Ac, &h->sc->coarse_bad, (VT*)h->tl_Ainv, h->stream);
     keep_coarse_in_l2(h, (size_t)nc * h->tl_ld * sizeof(VT));
     h->tl_ready = true;
     h->tl_refreshes++;
@@ -1062,9 +1073,11 @@ void coarse_rate_check(SorsHandle* h, bool refreshed, double* ref_rate, bool* re
 
 // A coarse operator built for the last solve (refreshed) is not kept when the
 // Hessian turns out to hold inverted elements or NaN: the one-launch PCG builds it
-// before the host has read the evaluation's scalars.
+// before the host has read the evaluation's scalars.  One of an indefinite Hessian is
+// zero (block Jacobi alone) and is built anew for the next Hessian.
 void coarse_state_check(SorsHandle* h, bool refreshed, bool* ready) {
     const DevScalars& sh = *h->sc_host;
+    if (refreshed && sh.coarse_bad) h->coarse_retry = true;
     if (refreshed && ((sh.status & kFlagInverted) || !(sh.gnorm2 == sh.gnorm2) || !(sh.rr == sh.rr) ||
                       !(sh.rz == sh.rz) || !(sh.pq == sh.pq)))
         *ready = false;
@@ -1516,8 +1529,9 @@ int build_resident_coarse(SorsHandle* h) {
     CK(cudaMemsetAsync(h->rc_Ac, 0, sizeof(double) * ((size_t)nc * nc + nc), h->stream));
     launch_range_galerkin<VT>(h->rc_npairs, h->rc_ab, h->rc_row0, h->row_ptr, h->col, (const VT*)h->H, h->rcargs,
                               h->rc_Ac, h->rc_diag, h->stream);
-    launch_coarse_invert(nc, h->rc_Ac, h->rc_diag, h->rc_work, h->stream);
-    launch_to_vt_perm<VT>(nc, h->rc_ld, h->rc_Ac, (VT*)h->rc_Ainv, h->stream);
+    int st = invert_coarse(h, nc, h->rc_Ac, h->rc_diag, h->rc_work);
+    if (st) return st;
+    launch_to_vt_perm<VT>(nc, h->rc_ld, h->rc_Ac, &h->sc->coarse_bad, (VT*)h->rc_Ainv, h->stream);
     h->rc_ready = true;
     h->rc_ref_rate = -1.0;
     h->tl_refreshes++;

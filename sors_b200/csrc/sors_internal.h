@@ -36,6 +36,7 @@ struct DevScalars {
     double rz, pq, alpha, beta, rr, tol2, bnorm2;
     int it, done, maxit, breakdown;
     int skip;            // the Newton iteration ends before its solve (NewtonForcing)
+    int coarse_bad;      // the last coarse matrix was indefinite (launch_coarse_invert)
     // MINRES (Lanczos vectors with Givens QR, minres.cu): gamma_{j-1},
     // gamma_j, delta_j, c_{j-1}, c_j, s_{j-1}, s_j and eta (the preconditioned
     // residual norm, signed); the solution update the last iteration left
@@ -318,15 +319,17 @@ void launch_coarse_galerkin_d(int npairs, const int* cpair_ptr, const int2* cpai
 template <typename HT>
 void launch_range_galerkin(int npairs, const int2* ab, const int* row0, const int* row_ptr, const int* col,
                            const HT* H, const CoarseArgs& c, double* Ac, double* diag, cudaStream_t st);
-// In-place inverse; diag: Ac's diagonal, work: coarse_work(nc) doubles.
-void launch_coarse_invert(int nc, double* Ac, const double* diag, double* work, cudaStream_t st);
+// In-place inverse; diag: Ac's diagonal, work: coarse_work(nc) doubles.  *bad becomes 1
+// where a pivot is below -neg of its unknown's diagonal: the matrix is indefinite.
+void launch_coarse_invert(int nc, double* Ac, const double* diag, double* work, double neg, int* bad, cudaStream_t st);
 constexpr int kCoarsePanel = 32;
 inline size_t coarse_work(int nc) { return (size_t)2 * kCoarsePanel * nc + kCoarsePanel * kCoarsePanel; }
+// in -> out, rows of ld entries; all zero where *bad is set
 template <typename VT>
-void launch_to_vt_pad(int nc, int ld, const double* in, VT* out, cudaStream_t st);
+void launch_to_vt_pad(int nc, int ld, const double* in, const int* bad, VT* out, cudaStream_t st);
 // column 6 b + m of `in` as column m nagg + b of `out` (the one-launch PCGs' order)
 template <typename VT>
-void launch_to_vt_perm(int nc, int ld, const double* in, VT* out, cudaStream_t st);
+void launch_to_vt_perm(int nc, int ld, const double* in, const int* bad, VT* out, cudaStream_t st);
 template <typename VT>
 void launch_coarse_restrict(const CoarseArgs& c, const VT* r, double* yc, cudaStream_t st);
 template <typename VT>
