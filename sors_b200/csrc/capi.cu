@@ -310,13 +310,13 @@ cudaError_t dzero(SorsHandle* h, void* dst, size_t bytes) {
     return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
 }
 
-// For the tests (sors_test_deny): how many device allocations and thread starts of this
-// thread fail next.
-thread_local int t_deny_allocs = 0, t_deny_threads = 0;
+// For the tests (sors_test_deny): how many of this thread's plan allocations and thread
+// starts fail next.
+thread_local int t_deny_plans = 0, t_deny_threads = 0;
 
 int dalloc(SorsHandle* h, void** p, size_t bytes) {
     if (bytes == 0) bytes = 16;
-    cudaError_t e = t_deny_allocs > 0 && t_deny_allocs-- ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+    cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
         *p = nullptr;
         return fail(SORS_ERR_OOM, std::string("device allocation of ") + std::to_string(bytes) +
@@ -325,6 +325,12 @@ int dalloc(SorsHandle* h, void** p, size_t bytes) {
     h->allocs.push_back(*p);
     h->bytes += bytes;
     return SORS_OK;
+}
+
+// The one-launch PCG's plan.
+int dalloc_plan(SorsHandle* h, char** p, size_t bytes) {
+    if (t_deny_plans > 0 && t_deny_plans--) return fail(SORS_ERR_OOM, "no room for the plan");
+    return dalloc(h, (void**)p, bytes);
 }
 
 template <typename T>
@@ -1324,7 +1330,7 @@ int plan_resident(SorsHandle* h) {
     const size_t cb = up(sizeof(double) * ((size_t)nc * nc + nc + coarse_work(nc))), vb = up((size_t)nc * nc * hs);
     char* base = nullptr;
     int st;
-    if ((st = dalloc(h, (void**)&base, zb + bb + 256 + cb + vb + host.size()))) return st;
+    if ((st = dalloc_plan(h, &base, zb + bb + 256 + cb + vb + host.size()))) return st;
     CK(cudaMemsetAsync(base, 0, zb + bb + 256, h->stream));
     h->res_zg = (unsigned long long*)base;
     h->res_box = (unsigned long long*)(base + zb);
@@ -1473,7 +1479,7 @@ int plan_stream(SorsHandle* h) {
                  cb = up(sizeof(double) * (nc * nc + nc + coarse_work((int)nc))), vb = up(nc * pl.ld * hs);
     char* base = nullptr;
     int st;
-    if ((st = dalloc(h, (void**)&base, zb + bb + ob + 256 + wb + fb + cb + vb + host.size()))) return st;
+    if ((st = dalloc_plan(h, &base, zb + bb + ob + 256 + wb + fb + cb + vb + host.size()))) return st;
     CK(cudaMemsetAsync(base, 0, zb + bb + ob + 256, h->stream));
     char* q = base;
     h->res_zg = (unsigned long long*)q; q += zb;
@@ -3277,11 +3283,14 @@ void sors_pcg_parts(int32_t n_nodes, int32_t n_elems, int32_t nodes_per_elem, in
     out[0] = p.form; out[1] = p.G; out[2] = p.A;
 }
 
-// Not part of the ABI: the calling thread's next device allocations and thread starts fail.
-void sors_test_deny(int32_t allocations, int32_t threads) {
-    t_deny_allocs = allocations;
+// Not part of the ABI: the calling thread's next plan allocations and thread starts fail.
+void sors_test_deny(int32_t plans, int32_t threads) {
+    t_deny_plans = plans;
     t_deny_threads = threads;
 }
+
+// Not part of the ABI: the form of the handle's one-launch PCG (pick_parts; 0: none).
+int32_t sors_test_pcg_form(const SorsHandle* h) { return h->parts_form; }
 
 // Not part of the ABI: the limit of the waits of the handle's one-launch PCG (0: a
 // single look, so that a wait runs out).
