@@ -1146,10 +1146,14 @@ Parts pick_parts(int N, int E, int nv, size_t hs, int sms, int max_blocks, bool 
     }
     // Grid: more blocks take fewer iterations (more, smaller aggregates) and longer
     // sums (over 148 blocks 2.2 us, over 64 1.4 us).  ms by number of blocks, 64 / 80 /
-    // 96 / 128 / 148: a step of 4,225 FP64 nodes 1.46 / 1.34 / 1.35 / 1.37 / 1.48, of
-    // 9,856 FP32 nodes 1.85 / 1.80 / 1.77 / 1.83 / 1.95; three SQP steps of 10,648 FP32
-    // nodes 12.2 / 12.9 / 12.2 / 13.7 / 14.5 (67: 13.4); an adjoint of 3,321 FP64 hex
-    // nodes 32.7 / 33.4 / 34.0 / 37.1 / 39.2.  Counts with many halvings bisect best.
+    // 96 / 128.  Below 4,000 nodes 64 are best, of tets and hexes, in a step and in an
+    // adjoint's projected solves (FP64): tets 3,600 nodes 1.23 / 1.23 / 1.25 / 1.27; hexes
+    // 2,500 1.29 / 1.30 / 1.34 / 1.38, 3,100 1.33 / 1.36 / 1.37 / 1.41; adjoints 2,511
+    // 18.9 / 19.0 / 19.7 / 21.1, 3,321 21.5 / 21.7 / 22.7 / 24.1, 3,700 20.9 / 21.3 / 21.9 /
+    // 22.7.  Above, 96: tets 4,225 1.46 / 1.34 / 1.31 / 1.35, 4,901 1.52 / 1.36 / 1.34 / 1.42,
+    // 6,076 1.57 / 1.60 / 1.46 / 1.55; hexes 4,477 1.56 / 1.50 / 1.52 / 1.66, 5,904 1.74 / 1.75
+    // / 1.70 / 1.78; 9,856 FP32 tet nodes 1.85 / 1.80 / 1.77 / 1.83 (148: 1.95).  Counts with
+    // many halvings bisect best.
     const int per = hs == 4 ? 160 : 128;  // rows that have a lane group each
     int G = gmax;
     for (int g : {64, 96, 128})
