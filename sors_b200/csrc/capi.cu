@@ -237,6 +237,7 @@ struct SorsHandle {
     bool rc_ready = false;
     double rc_ref_rate = 0.0;
     bool coarse_retry = false;          // the coarse operator was left out: build it for the next Hessian
+    double hess_c = 0.0, coarse_c = 0.0;  // inertia coefficient of H, and of the Hessian of the coarse operator
     int tl_req = 0;  // settings.two_level as given (2: where it pays)
 
     double prev_gnorm = -1.0;
@@ -769,7 +770,15 @@ int eval_system(SorsHandle* h, double dt, bool want_hess, AsmMode mode = kAsmSte
     int st = compute_external(h);
     if (st) return st;
     (want_hess ? h->n_hess_evals : h->n_grad_evals)++;
-    if (want_hess && h->coarse_retry) h->rc_ready = h->tl_ready = h->coarse_retry = false;
+    if (want_hess) {
+        // Inertia four times that of the coarse operator's Hessian (a step half as long), or a
+        // quarter of it: an operator of other proportions costs iterations (a static solve's
+        // took 389 a step of 0.1 ms, block Jacobi 9), and the first solves that the check of
+        // the rate could compare with are its own.
+        h->hess_c = inertia_coef(h, dt);
+        const bool other = h->hess_c > 4.0 * h->coarse_c || h->coarse_c > 4.0 * h->hess_c;
+        if (h->coarse_retry || other) h->rc_ready = h->tl_ready = h->coarse_retry = false;
+    }
     const int project = h->force_project >= 0 ? h->force_project
                         : (h->s.project_spd == 2 ? (h->proj_fallback ? 1 : 0) : h->s.project_spd);
     AsmArgs<HT> a = asm_args<HT>(h, dt, want_hess, mode, project);
@@ -1039,6 +1048,7 @@ int ensure_two_level(SorsHandle* h) {
 // Inverts a coarse matrix in place; sc->coarse_bad says that it was indefinite (beyond
 // what rounding of the Hessian's values makes of a singular one).
 int invert_coarse(SorsHandle* h, int nc, double* Ac, const double* diag, double* work) {
+    h->coarse_c = h->hess_c;
     CK(cudaMemsetAsync(&h->sc->coarse_bad, 0, sizeof(int), h->stream));
     launch_coarse_invert(nc, Ac, diag, work, mixed(h) ? 1e-5 : 1e-10, &h->sc->coarse_bad, h->stream);
     return SORS_OK;
